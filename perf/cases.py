@@ -53,7 +53,7 @@ def listed():
         # active-space triples
         ('ccsdt_act_32', _case('resident', 'CCSDt', 32, 7, 7, its=DIIS, act_occ=2, act_unocc=5)),
         # quadruples
-        ('ccsdtq_14', _case('resident', 'CCSDTQ', 14, 4, 4, its=2, rhf=True)),
+        ('ccsdtq_14', _case('resident', 'CCSDTQ', 14, 4, 4, rhf=True)),
         # left CCSD and CR-CC(2,3) of the 32-orbital benchmark molecule
         ('left_32', _case('left', 'CR-CC(2,3)', 32, 7, 7)),
     ]
@@ -94,7 +94,7 @@ def draw(rng):
         orbs = rng.randint(9, 14)
         occ = rng.choice((3, 4))
         opened = rng.choice((0, 1))
-        return _case('resident', 'CCSDTQ', orbs, occ, occ - opened, its=2, rhf=opened == 0 and rng.random() < 0.5)
+        return _case('resident', 'CCSDTQ', orbs, occ, occ - opened, rhf=opened == 0 and rng.random() < 0.5)
     orbs = rng.randint(12, 34)
     return _case('left', 'CR-CC(2,3)', orbs, max(3, orbs // 5), max(3, orbs // 5), its=rng.randint(4, 6))
 
