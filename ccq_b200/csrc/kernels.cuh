@@ -122,6 +122,31 @@ void launch_gett_f64(const GettArgs &a, int a_kmajor, int b_kmajor, cudaStream_t
 void launch_zero_view(double *C, const int *offm, const int *offn, int M, int N, cudaStream_t s);
 void launch_assemble(const AsmArgs &a, cudaStream_t s);
 
+// One block of a launch over many small contractions (multi.cu): an output tile and a K range of one of them,
+// C[cm[i] + cn[j]] (+)= alpha sum_k A[am[i] + ak[k]] B[bn[j] + bk[k]] for i < m, j < n, k < K.
+constexpr int MULTI_K = 256;   // longest K range of an item
+constexpr int MI_ADD = 1, MI_KSPLIT = 2, MI_NFAST = 4;   // add into C; warps split K; C contiguous along j
+constexpr int MI_VA = 8, MI_VB = 16;                     // 16-byte operand loads (as GettArgs::vec_a, vec_b)
+constexpr int MI_SHAPE = 8;    // flags >> MI_SHAPE: tile shape, below
+// 0..3: one warp's tile is 16 x 16, 32 x 8, 32 x 16, 16 x 32; 4..7: 64 x 64 of a block (+2: A k-major, +1: B
+// k-major); 8: one column (n = 1) and a few k; 9: copy or zero
+constexpr int MS_64 = 4, MS_VEC = 8, MS_COPY = 9;
+constexpr int MULTI_VEC_ROWS = 512, MULTI_VEC_K = 16;
+inline void multi_shape(int shape, int &rows, int &cols) {
+    rows = shape == MS_VEC ? MULTI_VEC_ROWS : shape >= MS_64 ? 64 : shape == 0 || shape == 3 ? 16 : 32;
+    cols = shape == MS_VEC ? 1 : shape >= MS_64 ? 64 : shape == 1 ? 8 : shape == 3 ? 32 : 16;
+}
+struct __align__(16) MultiItem {
+    const double *A, *B;
+    double *C;
+    const int *am, *bn, *ak, *bk, *cm, *cn;
+    double alpha;
+    int m, n, k, flags;
+};
+inline bool multi_is64(const MultiItem &it) { return it.flags >> MI_SHAPE >= MS_64 && it.flags >> MI_SHAPE < MS_VEC; }
+void launch_gett_multi(const MultiItem *items, int n, bool tiles64, cudaStream_t s);   // items of one kind
+cudaError_t preload_multi();
+
 // Batched launches over the contexts of many independent solves (one plan operation of every
 // context at once).  owner[i] is the context of entry i; entries of contexts with active[owner[i]]
 // zero do nothing.  GETTs: 64 x 64 tiles, split into K slices of the entry's kchunk (slices add into

@@ -125,6 +125,9 @@ struct Op {
     int split_choice = -1;     // -1 by shape (split_eligible); autotuned: 0 DMMA, 1 per-tile split kernel, 2 persistent
     int split_ws = 0;          // slicing workspace of a split GETT (0: the context's first; see split_pool)
     bool frozen = false;       // in a T3 / T4 phase of an externally corrected solve: not run
+    bool small = false;        // small enough for a launch shared with other contractions (small_gett)
+    int origin = -1;           // CCSDt: the plan operation this piece of a contraction came from
+    std::vector<GettSeg> hsegs;   // terms of a grouped launch (leader only)
     std::vector<size_t> group_ops;   // every op of a grouped launch (leader only; members are skipped)
     std::vector<int> hcm, hcn; // output offset tables (grouping key)
     AsmArgs asmargs{};
@@ -252,6 +255,26 @@ struct DevBuf {
     std::vector<long long> shape, stride;
     long long numel = 0;
     std::vector<std::vector<int>> groups;
+    bool zeroed = false;   // set to zero at the start of its run range; its writers only add (see plan_zeroed)
+};
+
+// A launch of a scheduled run: one plan operation, many small contractions together, or the zeroing of the
+// range's accumulation buffers.
+struct SchedNode {
+    enum Kind { OP, MULTI, CLEAR } kind = OP;
+    size_t op = 0;                  // OP
+    size_t item0 = 0, nitems = 0;   // MULTI
+    bool tiles64 = false;           // MULTI: 64 x 64 tiles (a kernel of their own)
+    std::vector<int> deps;          // earlier nodes it waits for
+    std::vector<std::string> first; // amplitude blocks it uses before any operation of the run writes them
+    bool sink = true;               // no later node waits for it
+};
+
+// Plan operations [from, to) as launches in an order that respects every dependency.
+struct Sched {
+    size_t from = 0, to = 0;
+    std::vector<SchedNode> nodes;
+    MultiItem *items = nullptr;
 };
 
 }  // namespace
@@ -295,6 +318,12 @@ struct ccq_b200_ctx {
     std::vector<cudaStream_t> side;
     std::vector<cudaEvent_t> opev;
     cudaEvent_t cap_ev = nullptr;
+    // scheduled runs by their first operation, and their device items (kept across rebuilds when they fit)
+    std::map<size_t, Sched> scheds;
+    std::map<size_t, std::pair<MultiItem *, size_t>> item_bufs;
+    bool forced = false;        // force_tile: every contraction on the pinned kernel family, none merged
+    // accumulation buffers of each run range, contiguous: [start of the range's first op] -> memory
+    std::map<size_t, std::pair<double *, long long>> zero_mem;
     long long t_dev = 0;        // t_vec elements resident on the device (T1+T2 for CCSD-level methods)
     bool trace_init = false;    // stage times of context creation on stderr
     std::chrono::steady_clock::time_point t_init0;
@@ -630,6 +659,7 @@ void restrict_to_active(ccq_b200_ctx *c, const ActiveSpace &as) {
         for (auto &po : pieces(side[0]))
             for (auto &pv : pieces(side[1])) {
                 Op q = o;
+                q.origin = (int)(&o - &c->plan.ops[0]);
                 q.filters = po;
                 q.filters.insert(q.filters.end(), pv.begin(), pv.end());
                 ops.push_back(q);
@@ -680,6 +710,125 @@ void trace_stamp(const ccq_b200_ctx *c, const char *what) {
     if (!c->trace_init) return;
     double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - c->t_init0).count();
     fprintf(stderr, "ccq_b200_init %-14s %8.2f ms\n", what, ms);
+}
+
+// ---------------------------------------------------------------------------
+// Small contractions.  Most of a sweep's contractions take less time than their launch; those are run
+// together, all that are ready at one time in one grid (csrc/multi.cu, build_sched below).
+// ---------------------------------------------------------------------------
+// M, N, K of a GETT from its views, before restrictions and filters
+void gett_extents(const ccq_b200_ctx *c, const Op &o, long long (&mnk)[3]) {
+    auto in = [](const ViewSpec &v, const std::string &l) {
+        for (auto &ax : v.axes)
+            if (ax.label == l) return true;
+        return false;
+    };
+    mnk[0] = mnk[1] = mnk[2] = 1;
+    std::map<std::string, int> seen;
+    for (auto &ax : o.a.axes)
+        if (!seen[ax.label]++) mnk[in(o.c, ax.label) ? 0 : 2] *= tok(c, ax.size);
+    for (auto &ax : o.b.axes)
+        if (in(o.c, ax.label) && !in(o.a, ax.label) && !seen[ax.label]++) mnk[1] *= tok(c, ax.size);
+}
+
+// A contraction shares a launch when its products take the chip about ten microseconds at most and its output is
+// small enough to be added into.  Of 120 / 300 / 400 MFLOP the higher limits are better where many contractions
+// of a few hundred MFLOP wait for each other (CCSDt at 32 orbitals 22.4 / 21.5 / 21.0 ms a pass, the left solve at 32
+// 15.7 / 13.2 / 13.1 ms) and cost 1-2 % at 24 orbitals (7.1 / 7.2 ms); a 40-orbital CCSDT sweep does not see them.
+constexpr double kSmallFlops = 400e6;
+constexpr long long kSmallOut = 1 << 20;
+bool small_gett(const long long (&mnk)[3]) {
+    return 2.0 * mnk[0] * mnk[1] * mnk[2] <= kSmallFlops && mnk[0] * mnk[1] <= kSmallOut;
+}
+
+// the run ranges of a plan: the sweep with its energy, and for CR-CC(2,3) plans the left solve's
+// preparation, its iteration, and the triples corrections
+std::vector<size_t> run_ranges(const ccq_b200_ctx *c) {
+    std::vector<size_t> r{0};
+    for (size_t i = 0; i < c->plan.ops.size(); ++i)
+        if (c->plan.ops[i].kind == OP_PHASE &&
+            (c->plan.ops[i].arg0 == "crcc" || c->plan.ops[i].arg0 == "lambda" || c->plan.ops[i].arg0 == "triplesA"))
+            r.push_back(i);
+    r.push_back(c->plan.ops.size());
+    return r;
+}
+
+// Accumulation buffers: the intermediates that only small contractions write, all before the first read and
+// all in one run range.  They live outside the phases' shared arena, contiguous per range, so that one memset
+// at the range's start zeroes them; their writers then only add, in any order and with any split of K.  At
+// most kZeroBytes per range, smallest first.
+constexpr long long kZeroBytes = 96LL << 20;
+std::map<std::string, double *> plan_zeroed(ccq_b200_ctx *c) {
+    struct Info {
+        bool ok = true, read = false;
+        int first = -1, origin = -1;
+        size_t range = 0;
+        long long numel = 0;
+    };
+    std::map<std::string, Info> info;
+    for (auto &b : c->plan.bufs) {
+        if (b.kind != "work" && b.kind != "hx") continue;
+        long long ne = 1;
+        for (auto &d : b.dims) ne *= tok(c, d);
+        info[b.name].numel = (ne + 31) / 32 * 32;
+    }
+    const std::vector<size_t> ranges = run_ranges(c);
+    size_t rg = 0;
+    for (size_t i = 0; i < c->plan.ops.size(); ++i) {
+        while (rg + 2 < ranges.size() && i >= ranges[rg + 1]) ++rg;
+        Op &o = c->plan.ops[i];
+        auto read = [&](const std::string &b) {
+            auto it = info.find(b);
+            if (it != info.end()) it->second.read = true;
+        };
+        if (o.kind == OP_GETT) {
+            long long mnk[3];
+            gett_extents(c, o, mnk);
+            // what may run in split precision keeps its own launch
+            const bool bulk = o.tag.size() > 2 && o.tag[0] == 'T' && (o.tag[1] == '3' || o.tag[1] == '4') &&
+                              mnk[0] >= 64 && mnk[1] >= 64 && mnk[2] >= 256;
+            o.small = small_gett(mnk) && !bulk;
+            read(o.a.buf);
+            read(o.b.buf);
+            auto it = info.find(o.c.buf);
+            if (it == info.end()) continue;
+            Info &f = it->second;
+            if (f.first < 0) {
+                f.first = (int)i;
+                f.origin = o.origin;
+                f.range = ranges[rg];
+                f.ok = f.ok && o.beta == 0;
+            } else if (o.beta == 0 && !(o.origin >= 0 && o.origin == f.origin)) {
+                f.ok = false;   // overwritten again
+            }
+            f.ok = f.ok && o.small && !f.read && f.range == ranges[rg];
+        } else if (o.kind == OP_ASM) {
+            for (auto &t : o.terms) read(t.second.buf);
+            if (info.count(o.block)) info[o.block].ok = false;
+        } else if (o.kind == OP_COPY || o.kind == OP_ZERO) {
+            read(o.arg1);
+            if (info.count(o.arg0)) info[o.arg0].ok = false;
+        }
+    }
+    std::map<size_t, std::vector<std::pair<long long, std::string>>> by_range;
+    for (auto &kv : info)
+        if (kv.second.ok && kv.second.first >= 0) by_range[kv.second.range].push_back({kv.second.numel, kv.first});
+    std::map<std::string, double *> out;
+    for (auto &br : by_range) {
+        std::sort(br.second.begin(), br.second.end());
+        long long total = 0;
+        size_t n = 0;
+        while (n < br.second.size() && 8 * (total + br.second[n].first) <= kZeroBytes) total += br.second[n++].first;
+        if (!total) continue;
+        double *mem = (double *)c->dalloc(sizeof(double) * total);
+        c->zero_mem[br.first] = {mem, total};
+        long long off = 0;
+        for (size_t k = 0; k < n; ++k) {
+            out[br.second[k].second] = mem + off;
+            off += br.second[k].first;
+        }
+    }
+    return out;
 }
 
 void instantiate(ccq_b200_ctx *c) {
@@ -777,11 +926,12 @@ void instantiate(ccq_b200_ctx *c) {
                         throw Error(CCQ_B200_EPLAN, t.second.buf + " read by assemble before written");
         }
     }
+    const std::map<std::string, double *> zero_ptr = plan_zeroed(c);
     std::map<std::string, long long> phase_fill;
     std::map<std::string, long long> work_off;
     long long arena = 0;
     for (auto &b : c->plan.bufs) {
-        if (b.kind != "work") continue;
+        if (b.kind != "work" || zero_ptr.count(b.name)) continue;
         long long ne = 1;
         for (auto &d : b.dims) ne *= tok(c, d);
         ne = (ne + 31) / 32 * 32;
@@ -804,7 +954,7 @@ void instantiate(ccq_b200_ctx *c) {
             std::map<std::string, int> parity;
             for (size_t k = 0; k < order.size(); ++k) parity[order[k].second] = (int)(k & 1);
             for (auto &b : c->plan.bufs) {
-                if (b.kind != "work") continue;
+                if (b.kind != "work" || zero_ptr.count(b.name)) continue;
                 const std::string ph = first_phase.count(b.name) ? first_phase[b.name] : "unused";
                 if (parity[ph]) work_off[b.name] += arena;
             }
@@ -824,6 +974,9 @@ void instantiate(ccq_b200_ctx *c) {
             d.ptr = tv_off[b.name] < c->t_dev ? c->tvec + tv_off[b.name] : nullptr;
         } else if (lv_off.count(b.name)) {
             d.ptr = c->lvec + lv_off[b.name];
+        } else if (zero_ptr.count(b.name)) {
+            d.ptr = zero_ptr.at(b.name);
+            d.zeroed = true;
         } else if (b.kind == "work") {
             d.ptr = arena_ptr + work_off[b.name];
         } else {
@@ -1357,6 +1510,7 @@ void instantiate(ccq_b200_ctx *c) {
                     }
                     lead.g.beta = c->plan.ops[cl[0].first].beta;
                     lead.g.nseg = (int)cl.size();
+                    lead.hsegs.assign(hsegs.begin() + (long)off, hsegs.end());
                     for (auto &mm : cl) lead.group_ops.push_back(mm.first);
                     lead.group_flops = fl;
                     lead.group_size = (int)cl.size();
@@ -1490,16 +1644,6 @@ void run_op(ccq_b200_ctx *c, Op &o, cudaStream_t st) {
     }
 }
 
-// ops[from, to) issued for stream capture as a DAG.  Every GETT waits only for
-// the GETTs it reads from, the last overwrite of its output and the earlier
-// readers of that output; beta = 1 writers of one buffer do not wait for each
-// other (their epilogues add with reductions).  Jacobi and copy assembles,
-// buffer copies and zeroing are nodes of the same kind (they overwrite their
-// output), so an assemble overlaps the next block's contractions that do not
-// read it.  The rest (split GETTs, whose slicing shares one workspace, and the
-// left-solve and CR-CC(2,3) kernels that accumulate scalars) is a barrier on
-// the capturing stream.  Independent contractions then run on side
-// streams at the same time.
 // every t_vec block resident on the device, and the last sweep op that writes it
 void prepare_copy_out(ccq_b200_ctx *c) {
     if (c->out_ready) return;
@@ -1607,45 +1751,445 @@ void copy_out_finish(ccq_b200_ctx *c, cudaStream_t st) {
     CK(cudaStreamWaitEvent(st, c->cjoin, 0));
 }
 
-void run_ops_dag(ccq_b200_ctx *c, size_t from, size_t to) {
-    // side streams of the captured dependency graph (CCQ_B200_DAG_STREAMS, 1..32, default 10: CCSDT-40
-    // split 13.63 / 12.81 / 12.51 / 12.55 ms per iteration with 3 / 6 / 10 / 16)
-    static const int NSIDE = [] {
-        const char *e = getenv("CCQ_B200_DAG_STREAMS");
-        const int v = e ? atoi(e) : 10;
-        return v >= 1 && v <= 32 ? v : 10;
-    }();
+// ---------------------------------------------------------------------------
+// Scheduled runs.  A range of plan operations becomes a list of launches: every operation has a start time from
+// the estimated durations of what it waits for, small contractions that start in the same time slot become one
+// launch (MULTI), and the launches are ordered by their starts.  An operation waits for the last writers of
+// what it reads, and for the readers and earlier writers of what it overwrites; operations that add into one
+// buffer do not wait for each other, nor do the disjoint pieces of one CCSDt contraction.  An estimated duration
+// is at least one slot, so whatever an operation waits for starts in an earlier slot and merging cannot close
+// a cycle.
+// ---------------------------------------------------------------------------
+constexpr int kSlot = 16;   // quarter microseconds: 4 us, about one small launch
+
+// what an operation reads, overwrites (or adds into) and accumulates
+struct OpIO {
+    std::vector<std::string> in;
+    std::string out, acc;
+    bool overwrite = true, barrier = false;
+};
+
+OpIO op_io(const ccq_b200_ctx *c, const Op &o, bool grouped) {
+    OpIO r;
+    switch (o.kind) {
+        case OP_GETT:
+            r.in = {o.a.buf, o.b.buf};
+            if (grouped)
+                for (size_t m : o.group_ops) {
+                    r.in.push_back(c->plan.ops[m].a.buf);
+                    r.in.push_back(c->plan.ops[m].b.buf);
+                }
+            r.out = o.c.buf;
+            // a grouped launch carries the beta of its first member (g.beta), not its own
+            r.overwrite = !o.g.beta || o.zero_first || o.g.K == 0;
+            break;
+        case OP_ASM:
+            for (auto &t : o.terms) r.in.push_back(t.second.buf);
+            r.in.push_back(o.block);
+            r.out = o.block;
+            if (o.asmargs.mode == 2) {
+                r.in.insert(r.in.end(), {"HDA", "HDB", "ECOR"});
+                r.acc = "LN";
+            }
+            break;
+        case OP_COPY:
+            r.in = {o.arg1};
+            r.out = o.arg0;
+            break;
+        case OP_ZERO:
+            r.out = o.arg0;
+            break;
+        case OP_LENERGY:
+            r.in = {"LN", "ECOR"};
+            r.out = "EL";
+            break;
+        case OP_CRCC:
+            r.in = {"M3" + o.arg0, "L3" + o.arg0, "HDA", "HDB", "H2AA", "H2AB", "H2BB"};
+            for (char q = 'A'; q <= 'D'; ++q)
+                for (const char *w : {"W1", "W2"}) r.in.push_back(std::string(w) + q);
+            r.acc = "E23";
+            break;
+        default:
+            r.barrier = true;
+    }
+    return r;
+}
+
+// The items of one contraction term.  64 x 64 tiles when both sides have at least kBigSide rows and the tiles fill
+// the chip; else the longer side goes to the 16-row side of the DMMA, the shorter one to its 8 columns.  K ranges
+// are at most MULTI_K, and half that while the grid is too small to fill the chip.
+constexpr long long kBigSide = 48, kBigTiles = 128;
+bool multi_big(const GettArgs &g) {
+    return std::min(g.M, g.N) >= kBigSide && g.K > 16 &&
+           ((g.M + 63) / 64) * ((g.N + 63LL) / 64) * ((g.K + 127) / 128) >= kBigTiles;
+}
+
+void add_items(std::vector<MultiItem> &out, const Op &o, const GettSeg &sg, bool add) {
+    const GettArgs &g = o.g;
+    bool sw = g.N > g.M;
+    const long long K = sg.K;
+    const bool big = multi_big(g);
+    if (big) sw = false;
+    const long long M = sw ? g.N : g.M, N = sw ? g.M : g.N;
+    int shape = N <= 8 ? 1 : N <= 16 ? 2 : 3;
+    const bool ks = K > 16 && !big;
+    if (ks && N > 8 && ((M + 31) / 32) * ((N + 31) / 32) * ((K + 127) / 128) < 64) shape = 0;
+    if (big) shape = MS_64 + 2 * o.akm + o.bkm;
+    if (N == 1 && K <= MULTI_VEC_K) shape = MS_VEC;
+    int rows, cols;
+    multi_shape(shape, rows, cols);
+    if (shape < MS_64 && !ks) rows *= 4;
+    const long long tm = (M + rows - 1) / rows, tn = (N + cols - 1) / cols;
+    long long kc = tm * tn * ((K + MULTI_K / 2 - 1) / (MULTI_K / 2)) <= 148 ? MULTI_K / 2 : MULTI_K;
+    const long long nk = std::max(1LL, (K + kc - 1) / kc);
+    kc = ((K + nk - 1) / nk + 15) / 16 * 16;
+    for (long long i = 0; i < tm; ++i)
+        for (long long j = 0; j < tn; ++j)
+            for (long long k = 0; k < K; k += kc) {
+                MultiItem it{};
+                it.A = sw ? sg.B : sg.A;
+                it.B = sw ? sg.A : sg.B;
+                it.C = g.C;
+                it.am = (sw ? sg.offB_n : sg.offA_m) + i * rows;
+                it.bn = (sw ? sg.offA_m : sg.offB_n) + j * cols;
+                it.ak = (sw ? sg.offB_k : sg.offA_k) + k;
+                it.bk = (sw ? sg.offA_k : sg.offB_k) + k;
+                it.cm = (sw ? g.offC_n : g.offC_m) + i * rows;
+                it.cn = (sw ? g.offC_m : g.offC_n) + j * cols;
+                it.alpha = sg.alpha;
+                it.m = (int)std::min<long long>(rows, M - i * rows);
+                it.n = (int)std::min<long long>(cols, N - j * cols);
+                it.k = (int)std::min(kc, K - k);
+                it.flags = (add ? MI_ADD : 0) | (ks ? MI_KSPLIT : 0) | ((g.c_nfast != 0) != sw ? MI_NFAST : 0) |
+                           (big && g.vec_a ? MI_VA : 0) | (big && g.vec_b ? MI_VB : 0) | shape << MI_SHAPE;
+                out.push_back(it);
+            }
+}
+
+Sched build_sched(ccq_b200_ctx *c, size_t from, size_t to) {
+    // operations as issued, in plan order
+    struct Unit {
+        size_t op;
+        bool merge = false, add = false, big = false;
+        std::vector<int> deps;
+        std::vector<std::string> first;
+        long long start = 0, dur = kSlot;
+        int node = -1;
+    };
+    struct State {
+        std::vector<int> writers, full, readers, pre;
+        int origin = -1;
+    };
+    std::vector<Unit> units;
+    std::map<std::string, int> id;
+    std::vector<State> st;
+    std::vector<const DevBuf *> buf;
+    std::vector<std::vector<int>> alias;   // other touched buffers in the same arena memory
+    auto buf_id = [&](const std::string &nm) {
+        auto it = id.find(nm);
+        if (it != id.end()) return it->second;
+        const int k = (int)st.size();
+        id[nm] = k;
+        st.emplace_back();
+        auto jt = c->bufs.find(nm);
+        const DevBuf *d = jt == c->bufs.end() ? nullptr : &jt->second;
+        buf.push_back(d);
+        alias.emplace_back();
+        if (d && d->ptr)
+            for (int q = 0; q < k; ++q)
+                if (buf[q] && buf[q]->ptr && buf[q]->ptr < d->ptr + std::max(d->numel, 1LL) &&
+                    d->ptr < buf[q]->ptr + std::max(buf[q]->numel, 1LL)) {
+                    alias[k].push_back(q);
+                    alias[q].push_back(k);
+                }
+        return k;
+    };
+    std::map<std::string, bool> amp;
+    for (auto &b : c->plan.bufs)
+        if (b.kind == "amp") amp[b.name] = true;
+    int barrier = -1;
+    bool clear = false;
+    for (size_t i = from; i < to; ++i) {
+        const Op &o = c->plan.ops[i];
+        if (o.kind == OP_PHASE || o.frozen) continue;
+        Unit u;
+        u.op = i;
+        bool zeroed = false;
+        if (o.kind == OP_GETT) {
+            if (o.g.M == 0 || o.g.N == 0) continue;
+            zeroed = c->bufs.at(o.c.buf).zeroed && !c->forced;
+            // terms of an accumulation buffer are issued one by one, other grouped terms by their leader
+            if (!zeroed && o.skip) continue;
+            if (o.g.K == 0 && (zeroed || o.g.beta)) continue;
+            u.add = zeroed || o.g.beta;
+            // a term that overwrites runs as one item per tile, so its K range is limited
+            u.merge = !c->forced && o.small && o.g.K > 0 && !use_split(c, o) &&
+                      (u.add || (o.group_ops.empty() && o.g.K <= MULTI_K));
+            if (!zeroed && !u.merge) u.add = false;
+            u.big = u.merge && multi_big(o.g);
+            clear = clear || zeroed;
+        } else if ((o.kind == OP_COPY || o.kind == OP_ZERO) && !c->forced) {
+            const DevBuf &d = c->bufs.at(o.arg0);
+            u.merge = d.numel <= 1 << 14 && (o.kind == OP_ZERO || c->bufs.at(o.arg1).numel == d.numel);
+        }
+        const OpIO io = op_io(c, o, !zeroed);
+        auto add = [&](const std::vector<int> &v) { u.deps.insert(u.deps.end(), v.begin(), v.end()); };
+        if (barrier >= 0) u.deps.push_back(barrier);
+        auto touch = [&](const std::string &nm) {
+            const int k = buf_id(nm);
+            if (amp.count(nm) && st[k].writers.empty()) u.first.push_back(nm);
+            return k;
+        };
+        auto overlaps = [&](int k) {
+            for (int q : alias[k]) {
+                add(st[q].writers);
+                add(st[q].readers);
+                add(st[q].full);
+            }
+        };
+        std::vector<int> ins;
+        for (auto &b : io.in) ins.push_back(touch(b));
+        if (!io.acc.empty()) buf_id(io.acc);
+        const int out = io.out.empty() ? -1 : touch(io.out), acc = io.acc.empty() ? -1 : buf_id(io.acc);
+        for (int k : ins) {
+            add(st[k].writers);
+            overlaps(k);
+        }
+        const bool piece = out >= 0 && !zeroed && io.overwrite && o.origin >= 0 && st[out].origin == o.origin &&
+                           o.group_ops.empty();
+        if (out >= 0) {
+            overlaps(out);
+            if (zeroed) {
+                // only adds, all before the first read
+            } else if (piece) {
+                add(st[out].pre);
+            } else {
+                add(st[out].readers);
+                add(io.overwrite ? st[out].writers : st[out].full);
+            }
+        }
+        if (acc >= 0) {
+            add(st[acc].full);
+            add(st[acc].readers);
+        }
+        // the slicing workspace of a split GETT: wait for its previous user
+        int ws = -1;
+        if (o.kind == OP_GETT && use_split(c, o)) {
+            ws = buf_id("@split" + std::to_string(c->split_pool.empty() ? 0 : o.split_ws));
+            add(st[ws].writers);
+        }
+        if (io.barrier)
+            for (int k = 0; k < (int)units.size(); ++k) u.deps.push_back(k);
+        std::sort(u.deps.begin(), u.deps.end());
+        u.deps.erase(std::unique(u.deps.begin(), u.deps.end()), u.deps.end());
+        for (int d : u.deps) u.start = std::max(u.start, units[d].start + units[d].dur);
+        if (!u.merge) {
+            // estimated duration in quarter microseconds: a launch, then the slower of arithmetic and traffic
+            double us = 5.0;
+            if (o.kind == OP_GETT) {
+                const double fl = o.group_size ? o.group_flops : 2.0 * o.g.M * o.g.N * o.g.K;
+                us += std::max(fl / 25e6, 8.0 * (2.0 * o.g.M * o.g.N + (double)(o.g.M + o.g.N) * o.g.K) / 4e6);
+            } else if (o.kind == OP_ASM) {
+                us += 8.0 * (double)c->bufs.at(o.block).numel * 2.0 / 3e6;
+            } else if (o.kind == OP_COPY) {
+                us += 16.0 * (double)c->bufs.at(o.arg0).numel / 4e6;
+            }
+            u.dur = std::max<long long>(kSlot, (long long)(us * 4.0));
+        }
+        const int me = (int)units.size();
+        for (int k : ins) st[k].readers.push_back(me);
+        if (out >= 0) {
+            State &s = st[out];
+            if (zeroed || (!io.overwrite && !piece)) {
+                s.writers.push_back(me);
+            } else if (piece) {
+                s.writers.push_back(me);
+                s.full.push_back(me);
+            } else {
+                s.pre = s.readers;
+                s.pre.insert(s.pre.end(), s.writers.begin(), s.writers.end());
+                s.writers.assign(1, me);
+                s.full.assign(1, me);
+                s.readers.clear();
+                s.origin = o.group_ops.empty() ? o.origin : -1;
+            }
+        }
+        if (acc >= 0) st[acc].writers.push_back(me);
+        if (ws >= 0) st[ws].writers.assign(1, me);
+        if (io.barrier) barrier = me;
+        units.push_back(std::move(u));
+    }
+    // nodes: single operations at their start, merged ones at their slot
+    Sched s;
+    s.from = from;
+    s.to = to;
+    struct Pre {
+        long long start;
+        std::vector<int> units;
+        bool merged;
+    };
+    std::vector<Pre> pre;
+    std::map<std::pair<long long, bool>, size_t> slot;
+    for (int k = 0; k < (int)units.size(); ++k) {
+        Unit &u = units[k];
+        if (!u.merge) {
+            pre.push_back({u.start, {k}, false});
+            continue;
+        }
+        const long long b = u.start / kSlot;
+        auto it = slot.find({b, u.big});
+        if (it == slot.end()) {
+            slot[{b, u.big}] = pre.size();
+            pre.push_back({b * kSlot, {k}, true});
+        } else {
+            pre[it->second].units.push_back(k);
+        }
+    }
+    std::vector<size_t> order(pre.size());
+    for (size_t k = 0; k < order.size(); ++k) order[k] = k;
+    std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return pre[a].start < pre[b].start; });
+    if (clear) {
+        SchedNode z;
+        z.kind = SchedNode::CLEAR;
+        s.nodes.push_back(z);
+    }
+    std::vector<MultiItem> items;
+    for (size_t pk : order) {
+        const int me = (int)s.nodes.size();
+        SchedNode n;
+        n.kind = pre[pk].merged ? SchedNode::MULTI : SchedNode::OP;
+        n.op = units[pre[pk].units[0]].op;
+        n.item0 = items.size();
+        n.tiles64 = units[pre[pk].units[0]].big;
+        bool zdep = false;
+        for (int k : pre[pk].units) {
+            Unit &u = units[k];
+            u.node = me;
+            for (int d : u.deps) n.deps.push_back(units[d].node);
+            n.first.insert(n.first.end(), u.first.begin(), u.first.end());
+            const Op &o = c->plan.ops[u.op];
+            if (o.kind == OP_GETT && c->bufs.at(o.c.buf).zeroed) zdep = zdep || !c->forced;
+            if (!pre[pk].merged) continue;
+            if (o.kind == OP_GETT) {
+                const GettArgs &g = o.g;
+                const bool one = o.group_ops.empty() || c->bufs.at(o.c.buf).zeroed;
+                if (one)
+                    add_items(items, o, GettSeg{g.A, g.B, g.offA_m, g.offA_k, g.offB_n, g.offB_k, g.K, g.alpha}, u.add);
+                else
+                    for (auto &sg : o.hsegs) add_items(items, o, sg, u.add);
+            } else {
+                const DevBuf &d = c->bufs.at(o.arg0);
+                const double *src = o.kind == OP_COPY ? c->bufs.at(o.arg1).ptr : nullptr;
+                for (long long x = 0, ne = std::max(d.numel, 1LL); x < ne; x += 1024) {
+                    MultiItem it{};
+                    it.A = src ? src + x : nullptr;
+                    it.C = d.ptr + x;
+                    it.m = (int)std::min(1024LL, ne - x);
+                    it.flags = MS_COPY << MI_SHAPE;
+                    items.push_back(it);
+                }
+            }
+        }
+        n.nitems = items.size() - n.item0;
+        // the longest items first, so that the launch does not end on one
+        auto cost = [](const MultiItem &it) {
+            const int shape = it.flags >> MI_SHAPE;
+            if (shape >= MS_VEC) return 0;
+            int rows, cols;
+            multi_shape(shape, rows, cols);
+            return rows * cols / 256 * ((it.k + 7) / 8) / (it.flags & MI_KSPLIT ? 4 : 1);
+        };
+        std::stable_sort(items.begin() + (long)n.item0, items.end(),
+                         [&](const MultiItem &x, const MultiItem &y) { return cost(x) > cost(y); });
+        if (zdep) n.deps.push_back(0);
+        s.nodes.push_back(n);
+    }
+    // direct dependencies only: those not reached through another one
+    const size_t nn = s.nodes.size(), words = (nn + 63) / 64;
+    std::vector<std::vector<uint64_t>> anc(nn, std::vector<uint64_t>(words, 0));
+    for (size_t k = 0; k < nn; ++k) {
+        SchedNode &n = s.nodes[k];
+        std::sort(n.deps.begin(), n.deps.end(), std::greater<int>());
+        n.deps.erase(std::unique(n.deps.begin(), n.deps.end()), n.deps.end());
+        std::vector<int> keep;
+        for (int d : n.deps) {
+            if (d < 0 || d >= (int)k) throw Error(CCQ_B200_EPLAN, "schedule out of order");
+            if (anc[k][d >> 6] >> (d & 63) & 1) continue;
+            keep.push_back(d);
+            s.nodes[d].sink = false;
+            for (size_t w = 0; w < words; ++w) anc[k][w] |= anc[d][w];
+            anc[k][d >> 6] |= 1ull << (d & 63);
+        }
+        n.deps = keep;
+    }
+    if (!items.empty()) {
+        auto &ib = c->item_bufs[from];
+        CK(cudaStreamSynchronize(c->stream));   // no earlier launch still reads them
+        if (ib.second < items.size()) ib = {(MultiItem *)c->dalloc(sizeof(MultiItem) * items.size()), items.size()};
+        CK(cudaMemcpy(ib.first, items.data(), sizeof(MultiItem) * items.size(), cudaMemcpyHostToDevice));
+        s.items = ib.first;
+    }
+    if (c->trace_init)
+        fprintf(stderr, "ccq_b200 schedule [%zu, %zu): %zu operations, %zu launches, %zu items\n", from, to,
+                units.size(), nn, items.size());
+    return s;
+}
+
+Sched &sched_for(ccq_b200_ctx *c, size_t from, size_t to) {
+    auto it = c->scheds.find(from);
+    if (it == c->scheds.end() || it->second.to != to) {
+        c->scheds[from] = build_sched(c, from, to);
+        return c->scheds[from];
+    }
+    return it->second;
+}
+
+void run_node(ccq_b200_ctx *c, const Sched &s, const SchedNode &n, cudaStream_t st) {
+    if (n.kind == SchedNode::MULTI) {
+        launch_gett_multi(s.items + n.item0, (int)n.nitems, n.tiles64, st);
+        ++c->launches;
+    } else if (n.kind == SchedNode::CLEAR) {
+        const auto &z = c->zero_mem.at(s.from);
+        CK(cudaMemsetAsync(z.first, 0, sizeof(double) * z.second, st));
+    } else {
+        run_op(c, c->plan.ops[n.op], st);
+    }
+}
+
+// The launches of plan operations [from, to) issued on the context's stream one after the other, or (dag, under
+// capture) on side streams with the dependencies as edges, so that independent launches run at the same time.
+void run_sched(ccq_b200_ctx *c, size_t from, size_t to, bool dag) {
+    const Sched &s = sched_for(c, from, to);
+    auto out_after = [&](const SchedNode &n, cudaStream_t st) {
+        if (n.kind == SchedNode::OP) copy_out_after(c, n.op, st);
+    };
+    if (!dag) {
+        for (auto &n : s.nodes) {
+            run_node(c, s, n, c->stream);
+            out_after(n, c->stream);
+        }
+        CK(cudaGetLastError());
+        return;
+    }
+    constexpr int NSIDE = 10;   // side streams (CCSDT-40 split 13.63 / 12.81 / 12.51 / 12.55 ms with 3 / 6 / 10 / 16)
     if (c->side.empty()) {
         c->side.resize(NSIDE);
         for (auto &st : c->side) CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&c->cap_ev, cudaEventDisableTiming));
     }
-    if (c->opev.size() < c->plan.ops.size()) {
-        size_t old = c->opev.size();
-        c->opev.resize(c->plan.ops.size(), nullptr);
-        for (size_t i = old; i < c->opev.size(); ++i) CK(cudaEventCreateWithFlags(&c->opev[i], cudaEventDisableTiming));
-    }
-    struct BufState {
-        std::vector<size_t> writers, full, readers;
+    auto events = [&](size_t n) {
+        for (size_t i = c->opev.size(); i < n; ++i) {
+            c->opev.push_back(nullptr);
+            CK(cudaEventCreateWithFlags(&c->opev[i], cudaEventDisableTiming));
+        }
     };
-    std::map<std::string, BufState> st;
-    std::vector<size_t> pending;
-    // CCQ_B200_DAG_SERIAL set: assembles, copies and zeroing are barriers (the earlier schedule, for comparison)
-    const bool serial_nodes = getenv("CCQ_B200_DAG_SERIAL") != nullptr;
-    cudaEvent_t gate = c->cap_ev;   // the last barrier (or the capture's start)
-    CK(cudaEventRecord(gate, c->stream));
-    int rr = 0;
-    std::vector<long long> last_on(NSIDE, -1);   // last node issued on each side stream since the last barrier
-    static const bool round_robin = getenv("CCQ_B200_DAG_ROUND_ROBIN") != nullptr;
-    auto join = [&]() {
-        for (size_t j : pending) CK(cudaStreamWaitEvent(c->stream, c->opev[j], 0));
-        pending.clear();
-        st.clear();
-        std::fill(last_on.begin(), last_on.end(), -1LL);
-    };
+    events(s.nodes.size());
+    CK(cudaEventRecord(c->cap_ev, c->stream));
+    std::map<std::string, cudaEvent_t> arrived;   // amplitude blocks on their way from the host
+    std::vector<cudaEvent_t> loose;
     if (c->host_in && from == 0) {
-        // the t_vec from the host, one node per amplitude block in t_vec order (T1, T2, then the T3 blocks)
-        // that the block's readers wait for (pseudo-op index ops.size() + k)
+        // the t_vec from the host, one copy per amplitude block in t_vec order (T1, T2, then the T3 blocks)
+        // that the block's readers wait for
         std::vector<std::pair<long long, std::string>> blk;
         for (auto &b : c->plan.bufs) {
             if (b.kind != "amp") continue;
@@ -1653,15 +2197,10 @@ void run_ops_dag(ccq_b200_ctx *c, size_t from, size_t to) {
             if (d.ptr && d.ptr >= c->tvec && d.ptr < c->tvec + c->t_dev) blk.push_back({d.ptr - c->tvec, b.name});
         }
         std::sort(blk.begin(), blk.end());
-        const size_t base = c->plan.ops.size();
-        if (c->opev.size() < base + blk.size() + 1) {
-            size_t old = c->opev.size();
-            c->opev.resize(base + blk.size() + 1, nullptr);
-            for (size_t i = old; i < c->opev.size(); ++i)
-                CK(cudaEventCreateWithFlags(&c->opev[i], cudaEventDisableTiming));
-        }
+        const size_t base = s.nodes.size();
+        events(base + blk.size() + 1);
         if (!c->istream) CK(cudaStreamCreateWithFlags(&c->istream, cudaStreamNonBlocking));
-        CK(cudaStreamWaitEvent(c->istream, gate, 0));
+        CK(cudaStreamWaitEvent(c->istream, c->cap_ev, 0));
         // every element of [0, t_dev) once: block k covers up to the next block's start
         long long lo = 0;
         for (size_t k = 0; k < blk.size(); ++k) {
@@ -1683,131 +2222,57 @@ void run_ops_dag(ccq_b200_ctx *c, size_t from, size_t to) {
             }
             lo = hi;
             CK(cudaEventRecord(c->opev[base + k], c->istream));
-            st[blk[k].second].writers.assign(1, base + k);
-            st[blk[k].second].full.assign(1, base + k);
-            pending.push_back(base + k);
+            arrived[blk[k].second] = c->opev[base + k];
+            loose.push_back(c->opev[base + k]);
         }
         if (blk.empty()) {
             CK(cudaMemcpyAsync(c->tvec, c->host_in, sizeof(double) * c->t_dev, cudaMemcpyHostToDevice, c->istream));
             CK(cudaEventRecord(c->opev[base], c->istream));
-            pending.push_back(base);
+            loose.push_back(c->opev[base]);
         }
     }
-    for (size_t i = from; i < to; ++i) {
-        Op &o = c->plan.ops[i];
-        if (o.kind == OP_PHASE || o.frozen) continue;
-        if (o.kind == OP_GETT && (o.skip || o.g.M == 0 || o.g.N == 0)) continue;
-        // Jacobi / copy assembles, buffer copies and zeroing are nodes too: each reads its term
-        // buffers (and its own block) and overwrites one buffer
-        const bool plain_node = !serial_nodes && ((o.kind == OP_ASM && o.asmargs.mode != 2) ||
-                                                  o.kind == OP_COPY || o.kind == OP_ZERO);
-        // a split GETT is a barrier only while every split GETT shares one slicing workspace
-        const bool splitop = o.kind == OP_GETT && use_split(c, o);
-        const bool barrier = (o.kind != OP_GETT && !plain_node) || (splitop && c->split_pool.empty());
-        if (barrier) {
-            join();
-            run_op(c, o, c->stream);
-            CK(cudaEventRecord(c->opev[i], c->stream));
-            gate = c->opev[i];
-            copy_out_after(c, i, c->stream);
-            continue;
-        }
-        std::vector<size_t> deps;
-        auto add = [&](const std::vector<size_t> &v) { deps.insert(deps.end(), v.begin(), v.end()); };
-        std::vector<std::string> ins;
-        std::string out;
-        bool overwrite = true;
-        if (o.kind == OP_GETT) {
-            ins = {o.a.buf, o.b.buf};
-            for (size_t m : o.group_ops) {
-                ins.push_back(c->plan.ops[m].a.buf);
-                ins.push_back(c->plan.ops[m].b.buf);
-            }
-            out = o.c.buf;
-            // a grouped launch carries the beta of its first member (g.beta), not its own
-            overwrite = !o.g.beta || o.zero_first || o.g.K == 0;
-        } else if (o.kind == OP_ASM) {
-            for (auto &t : o.terms) ins.push_back(t.second.buf);
-            ins.push_back(o.block);
-            out = o.block;
-        } else if (o.kind == OP_COPY) {
-            ins = {o.arg1};
-            out = o.arg0;
-        } else {
-            out = o.arg0;
-        }
-        // the Z/X work buffers of different block phases share one arena: an access also waits for
-        // every earlier access to a buffer whose memory overlaps
-        auto alias_deps = [&](const std::string &nm) {
-            auto it = c->bufs.find(nm);
-            if (it == c->bufs.end() || !it->second.ptr) return;
-            const double *lo = it->second.ptr, *hi = lo + std::max(it->second.numel, 1LL);
-            for (auto &kv : st) {
-                if (kv.first == nm) continue;
-                auto jt = c->bufs.find(kv.first);
-                if (jt == c->bufs.end() || !jt->second.ptr) continue;
-                const double *l2 = jt->second.ptr, *h2 = l2 + std::max(jt->second.numel, 1LL);
-                if (l2 < hi && lo < h2) {
-                    add(kv.second.writers);
-                    add(kv.second.readers);
-                    add(kv.second.full);
-                }
-            }
-        };
-        for (auto &b : ins) {
-            add(st[b].writers);
-            alias_deps(b);
-        }
-        alias_deps(out);
-        // the slicing workspace of a split GETT: wait for its previous user
-        const std::string wsname = splitop ? "@split" + std::to_string(o.split_ws) : std::string();
-        if (splitop) {
-            add(st[wsname].writers);
-            add(st[wsname].readers);
-        }
-        BufState &cs = st[out];
-        add(cs.readers);
-        add(overwrite ? cs.writers : cs.full);
-        std::sort(deps.begin(), deps.end());
-        deps.erase(std::unique(deps.begin(), deps.end()), deps.end());
-        // a captured stream orders its operations, so the stream chosen adds an edge from its last node:
-        // take the stream whose last node is the latest of this node's dependencies (a true edge), else
-        // the stream whose last node is the oldest (round robin when CCQ_B200_DAG_ROUND_ROBIN is set)
-        int si = rr++ % NSIDE;
-        if (!round_robin) {
-            int best = -1;
+    std::vector<int> last_on(NSIDE, -1);   // last node issued on each side stream
+    for (int i = 0; i < (int)s.nodes.size(); ++i) {
+        const SchedNode &n = s.nodes[i];
+        // a captured stream orders its operations, so the stream chosen adds an edge from its last node: take
+        // the stream whose last node is the latest of this node's dependencies (a true edge), else the stream
+        // whose last node is the oldest
+        int si = -1;
+        for (int q = 0; q < NSIDE; ++q)
+            if (last_on[q] >= 0 && std::find(n.deps.begin(), n.deps.end(), last_on[q]) != n.deps.end() &&
+                (si < 0 || last_on[q] > last_on[si]))
+                si = q;
+        if (si < 0)
             for (int q = 0; q < NSIDE; ++q)
-                if (last_on[q] >= 0 && std::binary_search(deps.begin(), deps.end(), (size_t)last_on[q]) &&
-                    (best < 0 || last_on[q] > last_on[best]))
-                    best = q;
-            if (best < 0)
-                for (int q = 0; q < NSIDE; ++q)
-                    if (best < 0 || last_on[q] < last_on[best]) best = q;
-            si = best;
-        }
-        last_on[si] = (long long)i;
+                if (si < 0 || last_on[q] < last_on[si]) si = q;
         cudaStream_t sd = c->side[si];
-        CK(cudaStreamWaitEvent(sd, gate, 0));
-        for (size_t d : deps) CK(cudaStreamWaitEvent(sd, c->opev[d], 0));
-        run_op(c, o, sd);
+        if (last_on[si] < 0) CK(cudaStreamWaitEvent(sd, c->cap_ev, 0));
+        for (int d : n.deps)
+            if (d != last_on[si]) CK(cudaStreamWaitEvent(sd, c->opev[d], 0));
+        for (auto &b : n.first) {
+            auto it = arrived.find(b);
+            if (it != arrived.end()) CK(cudaStreamWaitEvent(sd, it->second, 0));
+        }
+        last_on[si] = i;
+        run_node(c, s, n, sd);
         CK(cudaEventRecord(c->opev[i], sd));
-        copy_out_after(c, i, sd);
-        pending.push_back(i);
-        if (splitop) {
-            st[wsname].writers.assign(1, i);
-            st[wsname].readers.clear();
-        }
-        for (auto &b : ins) st[b].readers.push_back(i);
-        if (overwrite) {
-            cs.writers.assign(1, i);
-            cs.full.assign(1, i);
-            cs.readers.clear();
-        } else {
-            cs.writers.push_back(i);
-        }
+        out_after(n, sd);
     }
-    join();
+    for (int i = 0; i < (int)s.nodes.size(); ++i)
+        if (s.nodes[i].sink) CK(cudaStreamWaitEvent(c->stream, c->opev[i], 0));
+    for (auto e : loose) CK(cudaStreamWaitEvent(c->stream, e, 0));
     CK(cudaGetLastError());
+}
+
+void run_ops(ccq_b200_ctx *c, size_t from, size_t to);
+
+// A range that is run once per solve (not captured): scheduled on the context's stream, or operation by
+// operation while profiling and with graphs off.
+void run_range(ccq_b200_ctx *c, size_t from, size_t to) {
+    if (c->use_graph && !c->profile)
+        run_sched(c, from, to, false);
+    else
+        run_ops(c, from, to);
 }
 
 void run_ops(ccq_b200_ctx *c, size_t from, size_t to) {
@@ -1862,14 +2327,12 @@ void sweep(ccq_b200_ctx *c) {
     if (c->use_graph && !c->profile) {
         if (!ge) {
             if (c->host_out || c->host_in) prepare_copy_in(c);
+            sched_for(c, 0, c->cc_end);   // built before the capture: it allocates and copies
             cudaGraph_t g;
             long long l0 = c->launches;
             CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
             try {
-                if (c->use_graph == 2)
-                    run_ops(c, 0, c->cc_end);
-                else
-                    run_ops_dag(c, 0, c->cc_end);
+                run_sched(c, 0, c->cc_end, c->use_graph == 1);
                 copy_out_finish(c, c->stream);
             } catch (...) {
                 cudaStreamEndCapture(c->stream, &g);
@@ -1898,22 +2361,27 @@ void drop_graphs(ccq_b200_ctx *c) {
     c->gexec_host_ptr = nullptr;
     c->gexec_host_in = nullptr;
     c->out_ready = false;
+    c->scheds.clear();
+}
+
+// kernels of one plan operation
+long long op_launches(const ccq_b200_ctx *c, const Op &o) {
+    if (o.frozen) return 0;
+    if (o.kind == OP_GETT && o.g.M && o.g.N && !o.skip)
+        return (o.zero_first || o.g.K == 0) + (o.g.K ? (use_split(c, o) ? split_launch_count(o.g, c->nslices) : 1) : 0);
+    return o.kind == OP_ASM ? 1 : 0;
 }
 
 long long count_sweep_launches(ccq_b200_ctx *c) {
     long long n = 0;
-    for (size_t i = 0; i < c->cc_end; ++i) {
-        const Op &o = c->plan.ops[i];
-        if (o.frozen) continue;
-        if (o.kind == OP_GETT && o.g.M && o.g.N && !o.skip) {
-            if (o.zero_first || o.g.K == 0) ++n;
-            if (o.g.K)
-                n += use_split(c, o)
-                         ? split_launch_count(o.g, c->nslices) : 1;
-        } else if (o.kind == OP_ASM) {
-            ++n;
-        }
+    if (c->use_graph && !c->profile) {
+        for (auto &nd : sched_for(c, 0, c->cc_end).nodes)
+            n += nd.kind == SchedNode::MULTI ? 1
+                 : nd.kind == SchedNode::CLEAR ? 0
+                                                  : op_launches(c, c->plan.ops[nd.op]);
+        return n;
     }
+    for (size_t i = 0; i < c->cc_end; ++i) n += op_launches(c, c->plan.ops[i]);
     return n;
 }
 
@@ -1994,6 +2462,7 @@ static int init_impl(const ccq_b200_dims *dims, const char *calc_type, const dou
         keep_pool_memory(c->device);
         CK(gett_f64_prepare());
         CK(preload_kernels((int)diis_space));
+        CK(preload_multi());
         c->calc_type = ct;
         c->rhf = rhf != 0;
         c->shift = shift;
@@ -2626,7 +3095,7 @@ int ccq_b200_lambda_init(ccq_b200_ctx *c, double e_cor) {
         CK(cudaMemcpy(c->bufs.at("ECOR").ptr, &e_cor, sizeof(double), cudaMemcpyHostToDevice));
         CK(cudaMemsetAsync(c->lvec, 0, sizeof(double) * c->l_size, c->stream));
         CK(cudaMemsetAsync(c->lring, 0, sizeof(double) * (size_t)(c->ds + 1) * c->l_size, c->stream));
-        run_ops(c, c->cc_end, c->lambda_op);
+        run_range(c, c->cc_end, c->lambda_op);
         CK(cudaStreamSynchronize(c->stream));
         return 0;
     } catch (const Error &e) {
@@ -2644,13 +3113,11 @@ int ccq_b200_lambda_iterate(ccq_b200_ctx *c, int64_t iter, double *e_left, doubl
         CK(cudaEventRecord(c->ev0, c->stream));
         if (c->use_graph && !c->profile) {
             if (!c->lgexec) {
+                sched_for(c, c->lambda_op, c->triples_op);
                 cudaGraph_t g;
                 CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
                 try {
-                    if (c->use_graph == 2)
-                        run_ops(c, c->lambda_op, c->triples_op);
-                    else
-                        run_ops_dag(c, c->lambda_op, c->triples_op);
+                    run_sched(c, c->lambda_op, c->triples_op, c->use_graph == 1);
                 } catch (...) {
                     cudaStreamEndCapture(c->stream, &g);
                     throw;
@@ -2712,7 +3179,7 @@ int ccq_b200_crcc23(ccq_b200_ctx *c, double *e) {
         CK(cudaSetDevice(c->device));
         CK(cudaEventRecord(c->ev0, c->stream));
         CK(cudaMemsetAsync(c->bufs.at("E23").ptr, 0, 4 * sizeof(double), c->stream));
-        run_ops(c, c->triples_op, c->plan.ops.size());
+        run_range(c, c->triples_op, c->plan.ops.size());
         CK(cudaEventRecord(c->ev1, c->stream));
         CK(cudaMemcpyAsync(e, c->bufs.at("E23").ptr, 4 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -2962,6 +3429,7 @@ int ccq_b200_set_active(ccq_b200_ctx *c, int64_t act_occ_b, int64_t act_unocc_a)
 int ccq_b200_force_tile(ccq_b200_ctx *c, int64_t tile) {
     if (!c) return fail(Error(CCQ_B200_EINVAL, "null context"));
     if (tile < 0 || tile > 6) return fail(Error(CCQ_B200_EINVAL, "force_tile: 0..6"));
+    c->forced = tile != 0;
     for (auto &o : c->plan.ops) {
         if (o.kind != OP_GETT || o.g.K == 0) continue;
         o.g.tile = (int)tile;

@@ -1,0 +1,84 @@
+"""Scheduled runs (small contractions sharing launches, T1 dressing in two passes) against the same operations one
+by one: two iterations from T = 0 in both graph modes equal the eager ones.
+
+Tolerance: every element is a sum of at most about 1e5 products of numbers below the block's largest, rounded in
+another order; 1e-12 of the largest amplitude is that sum's FP64 rounding with room for two iterations."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+T12 = ('T1A', 'T1B', 'T2A', 'T2B', 'T2C')
+
+
+def _shapes(d, names):
+    out = {}
+    for b in names:
+        n, nb = int(b[1]), 'ABCDE'.index(b[2])
+        out[b] = (d.oa,) * (n - nb) + (d.ob,) * nb + (d.va,) * (n - nb) + (d.vb,) * nb
+    return out
+
+
+def _context(method, norb, occ_a, occ_b, froz, rhf=False, active=None):
+    from ccq_b200 import integrals as I
+    from ccq_b200 import lib, synth
+    h, e2, _ = synth.generate(synth.SynthSpec(norb, 2 * occ_b, 2 * norb, 0.03, 77 + norb))
+    fa, fb = I.fock(h, e2, occ_a, occ_b)
+    v = I.spin_blocks(e2, froz)
+    return lib.Context(froz, occ_a, occ_b, norb, method, fa, fb, *v, rhf=rhf, shift=0.5, active=active), \
+        I.Dims(froz, occ_a, occ_b, norb)
+
+
+def _modes(ctx, names, shapes, iterate=None):
+    res = []
+    for mode in (0, 1, 2):
+        ctx.use_graph(mode)
+        for b in names:
+            ctx.set_block(b, np.zeros(shapes[b]))
+        hist = [ctx.iterate(it)[:2] for it in (1, 2)]
+        res.append((np.array(hist), {b: ctx.get_block(b, shapes[b]) for b in names}))
+    return res
+
+
+@pytest.mark.parametrize('method,norb,occ_a,occ_b,froz,rhf', [
+    ('CCSD', 4, 2, 1, 0, False),      # items of one row
+    ('CCSD', 9, 4, 3, 1, False),      # odd extents, frozen core
+    ('CCSD', 17, 8, 8, 0, True),      # eight occupied: one tile exactly
+    ('CCSD', 21, 9, 9, 0, False),     # nine occupied: a second, nearly empty tile
+    ('CCSD', 30, 13, 11, 1, False),
+    ('CCSD', 40, 17, 17, 0, False),   # 24 occupied orbitals held per lane
+    ('CCSD', 44, 25, 25, 0, False),   # beyond what the dressing passes hold: the separate transforms
+    ('CCSDT', 9, 3, 2, 0, False),
+    ('CCSDT', 14, 4, 4, 0, True),
+    ('CCSDTQ', 8, 4, 3, 0, False),
+])
+def test_scheduled_run_equals_operations(method, norb, occ_a, occ_b, froz, rhf):
+    ctx, d = _context(method, norb, occ_a, occ_b, froz, rhf)
+    names = T12 + (('T3A', 'T3B', 'T3C', 'T3D') if method != 'CCSD' else ()) + \
+        (('T4A', 'T4B', 'T4C', 'T4D', 'T4E') if method == 'CCSDTQ' else ())
+    shapes = _shapes(d, names)
+    names = tuple(b for b in names if np.prod(shapes[b]))
+    ref, *others = _modes(ctx, names, shapes)
+    scale = max(np.abs(x).max() for x in ref[1].values())
+    assert np.isfinite(scale) and scale > 0
+    for hist, t in others:
+        np.testing.assert_allclose(hist, ref[0], rtol=1e-11)
+        for b in names:
+            np.testing.assert_allclose(t[b], ref[1][b], atol=1e-12 * scale, rtol=0, err_msg=b)
+    ctx.close()
+
+
+def test_scheduled_active_space_and_pinned_kernel():
+    """CCSDt (pieces of one contraction share an output) and force_tile (nothing merged) take the same steps."""
+    ctx, d = _context('CCSDt', 12, 4, 4, 0, active=(2, 7))
+    names = T12 + ('T3A', 'T3B', 'T3C', 'T3D')
+    shapes = _shapes(d, names)
+    ref, *others = _modes(ctx, names, shapes)
+    ctx.force_tile(1)
+    others += _modes(ctx, names, shapes)
+    scale = max(np.abs(x).max() for x in ref[1].values())
+    for hist, t in others:
+        np.testing.assert_allclose(hist, ref[0], rtol=1e-11)
+        for b in names:
+            np.testing.assert_allclose(t[b], ref[1][b], atol=1e-12 * scale, rtol=0, err_msg=b)
+    ctx.close()
