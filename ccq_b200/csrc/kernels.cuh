@@ -147,6 +147,18 @@ inline bool multi_is64(const MultiItem &it) { return it.flags >> MI_SHAPE >= MS_
 void launch_gett_multi(const MultiItem *items, int n, bool tiles64, cudaStream_t s);   // items of one kind
 cudaError_t preload_multi();
 
+// T1 dressing of one two-electron block v0[p][q][r][s] (n^4) into v (dress.cu): t1 [o1][n - o1] belongs to the
+// first and third index, t2 [o2][n - o2] to the second and fourth.  dress_fits: the block is
+// large enough to gain and the kernels' registers and shared memory hold its occupied orbitals.
+struct DressArgs {
+    const double *v0, *t1, *t2;
+    double *v;
+    int n, o1, o2;
+};
+bool dress_fits(const DressArgs &d);
+cudaError_t dress_prepare();   // shared-memory limits on the current device
+int launch_dress(const DressArgs &d, cudaStream_t s);   // returns the number of launches
+
 // Batched launches over the contexts of many independent solves (one plan operation of every
 // context at once).  owner[i] is the context of entry i; entries of contexts with active[owner[i]]
 // zero do nothing.  GETTs: 64 x 64 tiles, split into K slices of the entry's kchunk (slices add into

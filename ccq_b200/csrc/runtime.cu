@@ -128,6 +128,10 @@ struct Op {
     bool small = false;        // small enough for a launch shared with other contractions (small_gett)
     int origin = -1;           // CCSDt: the plan operation this piece of a contraction came from
     std::vector<GettSeg> hsegs;   // terms of a grouped launch (leader only)
+    // T1 dressing of a two-electron block as one node of a scheduled run: its copy leads (dress), its four
+    // transforms follow (dressed); operation by operation they run on their own
+    bool dress = false, dressed = false;
+    DressArgs dargs{};
     std::vector<size_t> group_ops;   // every op of a grouped launch (leader only; members are skipped)
     std::vector<int> hcm, hcn; // output offset tables (grouping key)
     AsmArgs asmargs{};
@@ -829,6 +833,61 @@ std::map<std::string, double *> plan_zeroed(ccq_b200_ctx *c) {
         }
     }
     return out;
+}
+
+// The copy and the four quarter transforms of one two-electron block's T1 dressing, recognised in the plan and
+// run as two passes over the block (csrc/dress.cu) by scheduled runs.
+void find_dressings(ccq_b200_ctx *c) {
+    auto &ops = c->plan.ops;
+    auto same = [](const ViewSpec &v, const std::string &text) {
+        const ViewSpec w = parse_view(text);
+        if (v.buf != w.buf || v.axes.size() != w.axes.size()) return false;
+        for (size_t k = 0; k < v.axes.size(); ++k)
+            if (v.axes[k].label != w.axes[k].label || v.axes[k].size != w.axes[k].size ||
+                v.axes[k].start != w.axes[k].start)
+                return false;
+        return true;
+    };
+    for (size_t i = 0; i < ops.size(); ++i) {
+        const std::string V = ops[i].arg0;
+        if (ops[i].kind != OP_COPY || (V != "VAA" && V != "VAB" && V != "VBB") || ops[i].arg1 != V + "0") continue;
+        const char A = V[1], B = V[2];
+        auto sp = [](char x, char s) { return std::string(1, x) + (char)(s - 'A' + 'a'); };
+        const std::string o1 = sp('o', A), v1 = sp('v', A), o2 = sp('o', B), v2 = sp('v', B);
+        const std::string T1 = std::string("T1") + A, T2 = std::string("T1") + B;
+        struct Want {
+            double alpha;
+            std::string c, a, b;
+        } want[4] = {
+            {-1.0, V + "[p:" + v1 + "@" + o1 + ",x1:n,x2:n,x3:n]", T1 + "[i:" + o1 + ",p:" + v1 + "]",
+             V + "[i:" + o1 + ",x1:n,x2:n,x3:n]"},
+            {-1.0, V + "[x0:n,p:" + v2 + "@" + o2 + ",x2:n,x3:n]", T2 + "[i:" + o2 + ",p:" + v2 + "]",
+             V + "[x0:n,i:" + o2 + ",x2:n,x3:n]"},
+            {1.0, V + "[x0:n,x1:n,r:" + o1 + ",x3:n]", T1 + "[r:" + o1 + ",e:" + v1 + "]",
+             V + "[x0:n,x1:n,e:" + v1 + "@" + o1 + ",x3:n]"},
+            {1.0, V + "[x0:n,x1:n,x2:n,r:" + o2 + "]", T2 + "[r:" + o2 + ",e:" + v2 + "]",
+             V + "[x0:n,x1:n,x2:n,e:" + v2 + "@" + o2 + "]"}};
+        // the next four operations of the phase that touch V are the transforms in this order
+        std::vector<size_t> found;
+        for (size_t j = i + 1; j < ops.size() && ops[j].kind != OP_PHASE && found.size() < 4; ++j) {
+            const Op &o = ops[j];
+            const bool touches = o.kind == OP_GETT ? o.a.buf == V || o.b.buf == V || o.c.buf == V
+                                                   : o.kind == OP_ASM || o.arg0 == V || o.arg1 == V;
+            if (!touches) continue;
+            const Want &w = want[found.size()];
+            if (o.kind != OP_GETT || o.alpha != w.alpha || o.beta != 1 || !o.restrict_groups.empty() ||
+                !o.filters.empty() || !same(o.c, w.c) || !same(o.a, w.a) || !same(o.b, w.b))
+                break;
+            found.push_back(j);
+        }
+        if (found.size() < 4) continue;
+        DressArgs d{c->bufs.at(V + "0").ptr, c->bufs.at(T1).ptr, c->bufs.at(T2).ptr, c->bufs.at(V).ptr, (int)c->n,
+                    (int)tok(c, o1), (int)tok(c, o2)};
+        if (!d.t1 || !d.t2 || !dress_fits(d)) continue;
+        ops[i].dress = true;
+        ops[i].dargs = d;
+        for (size_t j : found) ops[j].dressed = true;
+    }
 }
 
 void instantiate(ccq_b200_ctx *c) {
@@ -1558,6 +1617,7 @@ void instantiate(ccq_b200_ctx *c) {
             signs_before += o.asmargs.nperm;
         }
     }
+    find_dressings(c);
     // ring and scratch
     c->ring = (double *)c->dalloc(sizeof(double) * (size_t)(c->ds + 1) * std::max(c->vec_size, 1LL));
     c->scratch = (double *)c->dalloc(sizeof(double) * 512);
@@ -1911,7 +1971,7 @@ Sched build_sched(ccq_b200_ctx *c, size_t from, size_t to) {
     bool clear = false;
     for (size_t i = from; i < to; ++i) {
         const Op &o = c->plan.ops[i];
-        if (o.kind == OP_PHASE || o.frozen) continue;
+        if (o.kind == OP_PHASE || o.frozen || (o.dressed && !c->forced)) continue;
         Unit u;
         u.op = i;
         bool zeroed = false;
@@ -1930,9 +1990,10 @@ Sched build_sched(ccq_b200_ctx *c, size_t from, size_t to) {
             clear = clear || zeroed;
         } else if ((o.kind == OP_COPY || o.kind == OP_ZERO) && !c->forced) {
             const DevBuf &d = c->bufs.at(o.arg0);
-            u.merge = d.numel <= 1 << 14 && (o.kind == OP_ZERO || c->bufs.at(o.arg1).numel == d.numel);
+            u.merge = !o.dress && d.numel <= 1 << 14 && (o.kind == OP_ZERO || c->bufs.at(o.arg1).numel == d.numel);
         }
-        const OpIO io = op_io(c, o, !zeroed);
+        OpIO io = op_io(c, o, !zeroed);
+        if (o.dress && !c->forced) io.in.insert(io.in.end(), {std::string("T1") + o.arg0[1], std::string("T1") + o.arg0[2]});
         auto add = [&](const std::vector<int> &v) { u.deps.insert(u.deps.end(), v.begin(), v.end()); };
         if (barrier >= 0) u.deps.push_back(barrier);
         auto touch = [&](const std::string &nm) {
@@ -1992,7 +2053,7 @@ Sched build_sched(ccq_b200_ctx *c, size_t from, size_t to) {
             } else if (o.kind == OP_ASM) {
                 us += 8.0 * (double)c->bufs.at(o.block).numel * 2.0 / 3e6;
             } else if (o.kind == OP_COPY) {
-                us += 16.0 * (double)c->bufs.at(o.arg0).numel / 4e6;
+                us += (o.dress ? 40.0 : 16.0) * (double)c->bufs.at(o.arg0).numel / 4e6;
             }
             u.dur = std::max<long long>(kSlot, (long long)(us * 4.0));
         }
@@ -2151,6 +2212,8 @@ void run_node(ccq_b200_ctx *c, const Sched &s, const SchedNode &n, cudaStream_t 
     } else if (n.kind == SchedNode::CLEAR) {
         const auto &z = c->zero_mem.at(s.from);
         CK(cudaMemsetAsync(z.first, 0, sizeof(double) * z.second, st));
+    } else if (c->plan.ops[n.op].dress && !c->forced) {
+        c->launches += launch_dress(c->plan.ops[n.op].dargs, st);
     } else {
         run_op(c, c->plan.ops[n.op], st);
     }
@@ -2378,7 +2441,7 @@ long long count_sweep_launches(ccq_b200_ctx *c) {
         for (auto &nd : sched_for(c, 0, c->cc_end).nodes)
             n += nd.kind == SchedNode::MULTI ? 1
                  : nd.kind == SchedNode::CLEAR ? 0
-                                                  : op_launches(c, c->plan.ops[nd.op]);
+                 : c->plan.ops[nd.op].dress && !c->forced ? 3 : op_launches(c, c->plan.ops[nd.op]);
         return n;
     }
     for (size_t i = 0; i < c->cc_end; ++i) n += op_launches(c, c->plan.ops[i]);
@@ -2463,6 +2526,7 @@ static int init_impl(const ccq_b200_dims *dims, const char *calc_type, const dou
         CK(gett_f64_prepare());
         CK(preload_kernels((int)diis_space));
         CK(preload_multi());
+        CK(dress_prepare());
         c->calc_type = ct;
         c->rhf = rhf != 0;
         c->shift = shift;

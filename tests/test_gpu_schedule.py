@@ -43,11 +43,17 @@ def _modes(ctx, names, shapes, iterate=None):
 @pytest.mark.parametrize('method,norb,occ_a,occ_b,froz,rhf', [
     ('CCSD', 4, 2, 1, 0, False),      # items of one row
     ('CCSD', 9, 4, 3, 1, False),      # odd extents, frozen core
-    ('CCSD', 17, 8, 8, 0, True),      # eight occupied: one tile exactly
-    ('CCSD', 21, 9, 9, 0, False),     # nine occupied: a second, nearly empty tile
-    ('CCSD', 30, 13, 11, 1, False),
-    ('CCSD', 40, 17, 17, 0, False),   # 24 occupied orbitals held per lane
-    ('CCSD', 44, 25, 25, 0, False),   # beyond what the dressing passes hold: the separate transforms
+    ('CCSD', 31, 8, 8, 0, True),      # the largest block that is dressed by separate transforms
+    # dressing in two passes: 4 and 6 occupied orbitals held per lane, odd extents, 8 (one tile exactly), 9
+    # (a second tile, nearly empty), 12, 16 with different spins, 24
+    ('CCSD', 32, 3, 3, 0, False),
+    ('CCSD', 34, 6, 5, 0, False),
+    ('CCSD', 33, 8, 8, 0, True),
+    ('CCSD', 37, 9, 9, 0, False),
+    ('CCSD', 36, 12, 11, 1, False),
+    ('CCSD', 35, 15, 13, 0, False),
+    ('CCSD', 40, 17, 17, 0, False),
+    ('CCSD', 44, 25, 25, 0, False),   # beyond what the dressing passes hold
     ('CCSDT', 9, 3, 2, 0, False),
     ('CCSDT', 14, 4, 4, 0, True),
     ('CCSDTQ', 8, 4, 3, 0, False),
