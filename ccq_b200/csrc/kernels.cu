@@ -1313,33 +1313,139 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-__global__ void sqdiff_kernel(const double *a, const double *b, long long n, double *out) {
+// The step that follows every sweep, one pass: the new vector into its ring slot (cur; in place when src == cur), the
+// squared distance from the previous slot (prev null: from zero) and, from the block that finishes last, the results of the
+// iteration straight into the host's pinned slots.  Bound by HBM for the large vectors (24 bytes per element; the copy
+// and the sum apart took 32: 0.34 -> 0.27 ms for the 67.3 M elements of 40 orbitals) and by launches for the small ones:
+// copy, memset, sum and two result copies were 25 us of a 150 us iteration.
+__global__ void __launch_bounds__(256) ring_step_kernel(const double *__restrict__ src, double *cur,
+                                                        const double *__restrict__ prev, long long n,
+                                                        double *partial, unsigned *count,
+                                                        const double *__restrict__ energy, double *host) {
     double acc = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        double d = (a ? a[i] : 0.0) - b[i];
+    const long long step = (long long)gridDim.x * blockDim.x;
+    const bool copy = src != cur;
+    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (; i + 3 * step < n; i += 4 * step) {
+        double v[4], p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            v[u] = src[i + u * step];
+            p[u] = prev ? prev[i + u * step] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (copy) cur[i + u * step] = v[u];
+            const double d = p[u] - v[u];
+            acc += d * d;
+        }
+    }
+    for (; i < n; i += step) {
+        const double v = src[i], d = (prev ? prev[i] : 0.0) - v;
+        if (copy) cur[i] = v;
         acc += d * d;
     }
     acc = warp_sum(acc);
     __shared__ double sh[32];
+    __shared__ bool last;
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x < 32) {
         double v = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
         v = warp_sum(v);
-        if (threadIdx.x == 0) atomicAdd(out, v);
+        if (threadIdx.x == 0) {
+            partial[blockIdx.x] = v;
+            __threadfence();
+            last = atomicAdd(count, 1u) == gridDim.x - 1;
+        }
+    }
+    __syncthreads();
+    if (!last) return;
+    // the blocks' sums in their order: the result does not depend on which block is last
+    __threadfence();
+    acc = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) acc += __ldcg(partial + b);
+    acc = warp_sum(acc);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double v = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += sh[w];
+        host[0] = *energy;
+        host[1] = v;
+        *count = 0;   // for the next launch
     }
 }
 
-void launch_sqdiff(const double *a, const double *b, long long n, double *out, cudaStream_t s) {
-    cudaMemsetAsync(out, 0, sizeof(double), s);
-    long long blocks = (n + 255) / 256;
-    if (blocks > 148 * 8) blocks = 148 * 8;
-    if (blocks < 1) blocks = 1;
-    sqdiff_kernel<<<(int)blocks, 256, 0, s>>>(a, b, n, out);
+void launch_ring_step(const double *src, double *cur, const double *prev, long long n, double *partial, unsigned *count,
+                      const double *energy, double *host, cudaStream_t s) {
+    const long long blocks = std::max(1LL, std::min<long long>((n + 1023) / 1024, RING_BLOCKS));
+    ring_step_kernel<<<(int)blocks, 256, 0, s>>>(src, cur, prev, n, partial, count, energy, host);
+}
+
+// Bordered DIIS system of construct_b_mat (diis.F90:159-242, the corner is -1
+// as in the reference) solved by LU with partial pivoting like dgesv, by one warp: lane j holds column j in shared
+// memory (lane ds + 1 the right-hand side), the multipliers of a column are formed side by side.
+__device__ void diis_solve_warp(const double *gram, int ds, double *coef, int *info, int *host_info) {
+    __shared__ double B[13][15];
+    const int lane = threadIdx.x & 31, n = ds + 1;
+    for (int x = lane; x < n * (n + 1); x += 32) {
+        const int i = x / (n + 1), j = x % (n + 1);
+        double v;
+        if (j == n) v = i == ds ? -1.0 : 0.0;
+        else if (i == ds || j == ds) v = -1.0;
+        else v = __ldcg(gram + (i <= j ? i * ds + j : j * ds + i));
+        B[i][j] = v;
+    }
+    __syncwarp();
+    int inf = 0;
+    for (int k = 0; k < n; ++k) {
+        int p = k;
+        double best = fabs(B[k][k]);
+        for (int i = k + 1; i < n; ++i)
+            if (fabs(B[i][k]) > best) {
+                best = fabs(B[i][k]);
+                p = i;
+            }
+        if (best == 0.0) {
+            inf = k + 1;
+            break;
+        }
+        __syncwarp();
+        if (p != k && lane <= n) {
+            const double t = B[k][lane];
+            B[k][lane] = B[p][lane];
+            B[p][lane] = t;
+        }
+        __syncwarp();
+        const double f = (lane > k && lane < n) ? B[lane][k] / B[k][k] : 0.0;
+        const double bk = lane <= n ? B[k][lane] : 0.0;
+        __syncwarp();
+        for (int i = k + 1; i < n; ++i) {
+            const double fi = __shfl_sync(0xffffffffu, f, i);
+            if (lane >= k && lane <= n) B[i][lane] -= fi * bk;
+        }
+        __syncwarp();
+    }
+    if (lane == 0) {
+        if (!inf) {
+            double c[13];
+            for (int i = n - 1; i >= 0; --i) {
+                double s = B[i][n];
+                for (int j = i + 1; j < n; ++j) s -= B[i][j] * c[j];
+                c[i] = s / B[i][i];
+            }
+            for (int i = 0; i < n; ++i) coef[i] = c[i];
+        }
+        *info = inf;
+        *host_info = inf;
+    }
 }
 
 template <int DS>
-__global__ void gram_kernel(const double *ring, long long stride, long long n, double *gram) {
+__global__ void gram_kernel(const double *ring, long long stride, long long n, double *gram, unsigned *count,
+                            double *coef, int *info, int *host_info) {
     double acc[DS][DS];
 #pragma unroll
     for (int i = 0; i < DS; ++i)
@@ -1372,79 +1478,35 @@ __global__ void gram_kernel(const double *ring, long long stride, long long n, d
                 if (threadIdx.x == 0) atomicAdd(&gram[i * DS + j], w);
             }
         }
+    // the block that finishes last solves the bordered system and leaves the matrix at zero for the next step
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x < 32) {
+        diis_solve_warp(gram, DS, coef, info, host_info);
+        __syncwarp();
+        for (int x = threadIdx.x; x < DS * DS; x += 32) gram[x] = 0.0;
+        if (threadIdx.x == 0) *count = 0;
+    }
 }
 
-void launch_diis_gram(const double *ring, long long stride, int ds, long long n, double *gram, cudaStream_t s) {
-    cudaMemsetAsync(gram, 0, sizeof(double) * ds * ds, s);
+void launch_diis_gram(const double *ring, long long stride, int ds, long long n, double *gram, unsigned *count,
+                      double *coef, int *info, int *host_info, cudaStream_t s) {
     long long blocks = (n + 255) / 256;
     if (blocks > 148 * 4) blocks = 148 * 4;
     if (blocks < 1) blocks = 1;
     switch (ds) {
 #define CASE(D) \
-    case D: gram_kernel<D><<<(int)blocks, 256, 0, s>>>(ring, stride, n, gram); break;
+    case D: gram_kernel<D><<<(int)blocks, 256, 0, s>>>(ring, stride, n, gram, count, coef, info, host_info); break;
         CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8) CASE(9) CASE(10) CASE(11) CASE(12)
 #undef CASE
         default: break;
     }
-}
-
-// Bordered DIIS system of construct_b_mat (diis.F90:159-242, the corner is -1
-// as in the reference) solved by LU with partial pivoting like dgesv.
-__global__ void diis_solve_kernel(const double *gram, int ds, double *coef, int *info) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int n = ds + 1;
-    double B[13][13];
-    double c[13];
-    for (int i = 0; i < ds; ++i)
-        for (int j = 0; j < ds; ++j) B[i][j] = (i <= j) ? gram[i * ds + j] : gram[j * ds + i];
-    for (int i = 0; i < n; ++i) {
-        B[i][ds] = -1.0;
-        B[ds][i] = -1.0;
-        c[i] = 0.0;
-    }
-    c[ds] = -1.0;
-    int inf = 0;
-    for (int k = 0; k < n; ++k) {
-        int p = k;
-        double best = fabs(B[k][k]);
-        for (int i = k + 1; i < n; ++i)
-            if (fabs(B[i][k]) > best) {
-                best = fabs(B[i][k]);
-                p = i;
-            }
-        if (best == 0.0) {
-            inf = k + 1;
-            break;
-        }
-        if (p != k) {
-            for (int j = 0; j < n; ++j) {
-                double t = B[k][j];
-                B[k][j] = B[p][j];
-                B[p][j] = t;
-            }
-            double t = c[k];
-            c[k] = c[p];
-            c[p] = t;
-        }
-        for (int i = k + 1; i < n; ++i) {
-            double f = B[i][k] / B[k][k];
-            for (int j = k; j < n; ++j) B[i][j] -= f * B[k][j];
-            c[i] -= f * c[k];
-        }
-    }
-    if (!inf) {
-        for (int i = n - 1; i >= 0; --i) {
-            double s = c[i];
-            for (int j = i + 1; j < n; ++j) s -= B[i][j] * c[j];
-            c[i] = s / B[i][i];
-        }
-        for (int i = 0; i < n; ++i) coef[i] = c[i];
-    }
-    *info = inf;
-}
-
-void launch_diis_solve(double *gram, int ds, double *coef, int *info, cudaStream_t s) {
-    diis_solve_kernel<<<1, 32, 0, s>>>(gram, ds, coef, info);
 }
 
 __global__ void diis_extrap_kernel(const double *ring, long long stride, int ds, long long n, const double *coef,
@@ -1484,8 +1546,7 @@ cudaError_t preload_kernels(int ds) {
     touch((const void *)zero_view_kernel);
     touch((const void *)f2c4_kernel);
     touch((const void *)fill_kernel);
-    touch((const void *)sqdiff_kernel);
-    touch((const void *)diis_solve_kernel);
+    touch((const void *)ring_step_kernel);
     touch((const void *)diis_extrap_kernel);
     touch((const void *)assemble_kernel<2, int>);
     touch((const void *)assemble_kernel<4, int>);

@@ -178,7 +178,11 @@ void launch_copy_batched(const BatchCopy *cp, int n, const int *owner, const int
 void launch_zero_views_batched(const GettArgs *args, int n, const int *owner, const int *active, cudaStream_t s);
 void launch_fill(double *p, double v, long long n, cudaStream_t s);
 void launch_f2c4(const double *f, double *out, long long n, cudaStream_t s);
-void launch_sqdiff(const double *a, const double *b, long long n, double *out, cudaStream_t s);
+// The new vector src into its ring slot cur, |prev - src|^2, and {*energy, that} into host[0..1] (pinned, mapped).
+// partial: RING_BLOCKS doubles; count: zero before the first launch, and again after each.
+constexpr int RING_BLOCKS = 148 * 8;
+void launch_ring_step(const double *src, double *cur, const double *prev, long long n, double *partial, unsigned *count,
+                      const double *energy, double *host, cudaStream_t s);
 
 // ccq's compressed CCSDt T3 (get_t_sizes_act): geometry of its ten sub-blocks inside the full T3
 // blocks of a T vector, and the gather / scatter between the two (csrc/ccsdt_layout.cu)
@@ -196,8 +200,10 @@ void t3act_geometry(long long froz, long long occ_a, long long occ_b, long long 
                     long long act_unocc_a, T3ActGeom &g);
 void launch_t3act_gather(const T3ActGeom &g, const double *tvec, double *cvec, cudaStream_t s);
 void launch_t3act_scatter(const T3ActGeom &g, const double *cvec, double *tvec, cudaStream_t s);
-void launch_diis_gram(const double *ring, long long stride, int ds, long long n, double *gram, cudaStream_t s);
-void launch_diis_solve(double *gram, int ds, double *coef, int *info, cudaStream_t s);
+// B matrix of the ring's differences and the bordered solve: coef[ds + 1], info (also to the pinned host_info).
+// gram (ds^2) and count are zero before the first launch, and again after each.
+void launch_diis_gram(const double *ring, long long stride, int ds, long long n, double *gram, unsigned *count,
+                      double *coef, int *info, int *host_info, cudaStream_t s);
 void launch_diis_extrap(const double *ring, long long stride, int ds, long long n, const double *coef, double *t,
                         cudaStream_t s);
 

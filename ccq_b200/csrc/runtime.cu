@@ -435,6 +435,29 @@ long long tok(const ccq_b200_ctx *c, const std::string &s) {
     return it->second;
 }
 
+// c->scratch: DIIS matrix, its coefficients, the ring step's partial sums; c->dinfo: DIIS status, block counters
+constexpr int kScratchGram = 8, kScratchCoef = 8 + 169, kScratchPartial = 512;
+
+// Ring write, residuum and results of an iteration, and on schedule the DIIS system, for the vector vec of length vs
+void ring_and_diis(ccq_b200_ctx *c, double *ring, const double *vec, long long vs, int64_t iter, const double *energy,
+                   bool diis, cudaStream_t st) {
+    const int ds = c->ds;
+    auto slot = [&](long long it) {
+        long long q = it % (ds + 1);
+        return q == 0 ? ds + 1 : q;
+    };
+    double *cur = ring + (slot(iter) - 1) * vs;
+    const double *prev = iter == 1 ? nullptr : ring + (slot(iter - 1) - 1) * vs;
+    c->hpin[2] = 0.0;
+    unsigned *count = reinterpret_cast<unsigned *>(c->dinfo) + 1;
+    launch_ring_step(vec ? vec : cur, cur, prev, vs, c->scratch + kScratchPartial, count, energy, c->hpin, st);
+    c->launches += 1;
+    if (!diis) return;
+    launch_diis_gram(ring, vs, ds, vs, c->scratch + kScratchGram, count + 1, c->scratch + kScratchCoef, c->dinfo,
+                     reinterpret_cast<int *>(c->hpin + 2), st);
+    c->launches += 1;
+}
+
 struct Resolved {
     double *base;
     std::map<std::string, long long> stride;   // per label
@@ -1620,7 +1643,7 @@ void instantiate(ccq_b200_ctx *c) {
     find_dressings(c);
     // ring and scratch
     c->ring = (double *)c->dalloc(sizeof(double) * (size_t)(c->ds + 1) * std::max(c->vec_size, 1LL));
-    c->scratch = (double *)c->dalloc(sizeof(double) * 512);
+    c->scratch = (double *)c->dalloc(sizeof(double) * (kScratchPartial + RING_BLOCKS));
     c->dinfo = (int *)c->dalloc(sizeof(int) * 4);
     CK(cudaStreamSynchronize(c->stream));
 }
@@ -2955,44 +2978,32 @@ int ccq_b200_energy(ccq_b200_ctx *c, double *e) {
 static void post_sweep(ccq_b200_ctx *c, int64_t iter, cudaStream_t st) {
     const int ds = c->ds;
     const long long vs = c->vec_size;
-    auto slot = [&](long long it) {
-        long long q = it % (ds + 1);
-        return q == 0 ? ds + 1 : q;
-    };
-    double *cur = c->ring + (slot(iter) - 1) * vs;
     const bool packed = c->cdiis && vs > c->vec_t12;   // CCSDt's compressed DIIS vector (not while T3 is held)
     if (packed) {
+        const long long q = iter % (ds + 1);
+        double *cur = c->ring + ((q == 0 ? ds + 1 : q) - 1) * vs;
         CK(cudaMemcpyAsync(cur, c->tvec, sizeof(double) * c->vec_t12, cudaMemcpyDeviceToDevice, st));
         launch_t3act_gather(c->geom, c->tvec, cur + c->vec_t12, st);
         c->launches += 1;
-    } else {
-        CK(cudaMemcpyAsync(cur, c->tvec, sizeof(double) * vs, cudaMemcpyDeviceToDevice, st));
     }
-    const double *prev = iter == 1 ? nullptr : c->ring + (slot(iter - 1) - 1) * vs;
-    launch_sqdiff(prev, cur, vs, c->scratch, st);
-    c->launches += 1;
-    const int diis = (iter % (ds + 1)) == 0;
+    const bool diis = (iter % (ds + 1)) == 0;
+    ring_and_diis(c, c->ring, packed ? nullptr : c->tvec, vs, iter, c->bufs.at("E").ptr, diis, st);
     if (diis) {
-        launch_diis_gram(c->ring, vs, ds, vs, c->scratch + 8, st);
-        launch_diis_solve(c->scratch + 8, ds, c->scratch + 8 + 169, c->dinfo, st);
         if (packed) {
-            launch_diis_extrap(c->ring, vs, ds, vs, c->scratch + 8 + 169, c->cvec, st);
+            launch_diis_extrap(c->ring, vs, ds, vs, c->scratch + kScratchCoef, c->cvec, st);
             CK(cudaMemcpyAsync(c->tvec, c->cvec, sizeof(double) * c->vec_t12, cudaMemcpyDeviceToDevice, st));
             launch_t3act_scatter(c->geom, c->cvec + c->vec_t12, c->tvec, st);
             c->launches += 2;
         } else {
-            launch_diis_extrap(c->ring, vs, ds, vs, c->scratch + 8 + 169, c->tvec, st);
+            launch_diis_extrap(c->ring, vs, ds, vs, c->scratch + kScratchCoef, c->tvec, st);
+            c->launches += 1;
         }
-        c->launches += 3;
         // the extrapolation rewrote T1 .. T3: the host copy is taken (again)
         if (double *dst = c->host_out ? c->host_out : c->diis_out)
             CK(cudaMemcpyAsync(dst, c->tvec, sizeof(double) * c->t_dev, cudaMemcpyDeviceToHost, st));
     }
     CK(cudaEventRecord(c->ev2, st));
-    CK(cudaMemcpyAsync(c->hpin, c->bufs.at("E").ptr, sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(c->hpin + 1, c->scratch, sizeof(double), cudaMemcpyDeviceToHost, st));
-    c->hpin[2] = 0.0;
-    if (diis) CK(cudaMemcpyAsync(c->hpin + 2, c->dinfo, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaGetLastError());
 }
 
 static void iterate_launch(ccq_b200_ctx *c, int64_t iter) {
@@ -3196,37 +3207,23 @@ int ccq_b200_lambda_iterate(ccq_b200_ctx *c, int64_t iter, double *e_left, doubl
         }
         CK(cudaEventRecord(c->ev1, c->stream));
         // ring, residuum and DIIS on the lambda vector (jacobi_iter on l_vec, src/solve_cc.f90:175-269)
-        const int ds = c->ds;
-        const long long vs = c->l_size;
-        auto slot = [&](long long it) {
-            long long q = it % (ds + 1);
-            return q == 0 ? ds + 1 : q;
-        };
-        double *cur = c->lring + (slot(iter) - 1) * vs;
-        CK(cudaMemcpyAsync(cur, c->lvec, sizeof(double) * vs, cudaMemcpyDeviceToDevice, c->stream));
-        const double *prev = iter == 1 ? nullptr : c->lring + (slot(iter - 1) - 1) * vs;
-        launch_sqdiff(prev, cur, vs, c->scratch, c->stream);
-        const int diis = (iter % (ds + 1)) == 0;
-        if (diis) {
-            launch_diis_gram(c->lring, vs, ds, vs, c->scratch + 8, c->stream);
-            launch_diis_solve(c->scratch + 8, ds, c->scratch + 8 + 169, c->dinfo, c->stream);
-            launch_diis_extrap(c->lring, vs, ds, vs, c->scratch + 8 + 169, c->lvec, c->stream);
-        }
+        const bool diis = (iter % (c->ds + 1)) == 0;
+        ring_and_diis(c, c->lring, c->lvec, c->l_size, iter, c->bufs.at("EL").ptr, diis, c->stream);
+        if (diis)
+            launch_diis_extrap(c->lring, c->l_size, c->ds, c->l_size, c->scratch + kScratchCoef, c->lvec, c->stream);
         CK(cudaEventRecord(c->ev2, c->stream));
-        double hs[2];
-        int info = 0;
-        CK(cudaMemcpyAsync(&hs[0], c->bufs.at("EL").ptr, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaMemcpyAsync(&hs[1], c->scratch, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        if (diis) CK(cudaMemcpyAsync(&info, c->dinfo, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaGetLastError());
         CK(cudaStreamSynchronize(c->stream));
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
         c->sweep_ms = ms;
         CK(cudaEventElapsedTime(&ms, c->ev0, c->ev2));
         c->iter_ms = ms;
+        int info = 0;
+        memcpy(&info, c->hpin + 2, sizeof(int));
         if (diis && info != 0) throw Error(CCQ_B200_ESINGULAR, "calc_diis: DIIS error in DGESV");
-        if (e_left) *e_left = hs[0];
-        if (res) *res = std::sqrt(std::sqrt(hs[1]));
+        if (e_left) *e_left = c->hpin[0];
+        if (res) *res = std::sqrt(std::sqrt(c->hpin[1]));
         if (did_diis) *did_diis = diis;
         return 0;
     } catch (const Error &e) {

@@ -88,3 +88,24 @@ def test_scheduled_active_space_and_pinned_kernel():
         for b in names:
             np.testing.assert_allclose(t[b], ref[1][b], atol=1e-12 * scale, rtol=0, err_msg=b)
     ctx.close()
+
+
+@pytest.mark.parametrize('ds', [1, 2, 7, 12])
+def test_diis_space(ds):
+    """Two DIIS steps (the bordered system at its smallest, at odd sizes and at its largest) follow ccq's iteration:
+    energies and residua of the dense oracle within the 1e-11 of the other trajectory tests."""
+    from ccq_b200 import integrals as I
+    from ccq_b200 import lib, synth
+    from oracle.densecc import DenseCC
+    h, e2, _ = synth.generate(synth.SynthSpec(6, 6, 12, 0.09, 5))
+    fa, fb = I.fock(h, e2, 3, 3)
+    v = I.spin_blocks(e2, 0)
+    n = min(2 * (ds + 1), 15) + 1
+    hist = DenseCC(fa, fb, *v, I.Dims(0, 3, 3, 6), 'CCSD').solve(diis_space=ds, max_iter=n, tol=0.0)[3]
+    ctx = lib.Context(0, 3, 3, 6, 'CCSD', fa, fb, *v, diis_space=ds)
+    ctx.use_graph(1)
+    got = [ctx.iterate(it) for it in range(1, n + 1)]
+    assert [g[2] for g in got] == [it % (ds + 1) == 0 for it in range(1, n + 1)]
+    np.testing.assert_allclose([g[0] for g in got], [x[0] for x in hist], atol=1e-11, rtol=0)
+    np.testing.assert_allclose([g[1] ** 2 for g in got], [x[2] ** 2 for x in hist], atol=1e-11, rtol=0)
+    ctx.close()
