@@ -1190,6 +1190,8 @@ template <int RK, typename Off>
 __global__ void __launch_bounds__(256, 4) assemble_kernel(AsmArgs a) {
     constexpr int CH = 128;
     __shared__ SmTerm<RK> st[CH];
+    gdc_launch();
+    gdc_wait();
     assemble_body<RK, Off, CH>(a, st, (long long)blockIdx.x * blockDim.x * ASM_EPT,
                                (long long)gridDim.x * blockDim.x * ASM_EPT);
 }
@@ -1254,21 +1256,22 @@ void launch_assemble(const AsmArgs &a, cudaStream_t s) {
     long long blocks = (a.total + 256 * ASM_EPT - 1) / (256 * ASM_EPT);
     if (blocks > 148 * 32) blocks = 148 * 32;
     if (blocks < 1) blocks = 1;
+    auto go = [&](auto kernel) { launch_after(blocks <= kEarlyBlocks, kernel, (unsigned)blocks, 256, 0, s, a); };
     if (a.off32) {
         switch (a.rank) {
-            case 2: assemble_kernel<2, int><<<(int)blocks, 256, 0, s>>>(a); break;
-            case 4: assemble_kernel<4, int><<<(int)blocks, 256, 0, s>>>(a); break;
-            case 6: assemble_kernel<6, int><<<(int)blocks, 256, 0, s>>>(a); break;
-            case 8: assemble_kernel<8, int><<<(int)blocks, 256, 0, s>>>(a); break;
+            case 2: go(assemble_kernel<2, int>); break;
+            case 4: go(assemble_kernel<4, int>); break;
+            case 6: go(assemble_kernel<6, int>); break;
+            case 8: go(assemble_kernel<8, int>); break;
             default: break;
         }
         return;
     }
     switch (a.rank) {
-        case 2: assemble_kernel<2, long long><<<(int)blocks, 256, 0, s>>>(a); break;
-        case 4: assemble_kernel<4, long long><<<(int)blocks, 256, 0, s>>>(a); break;
-        case 6: assemble_kernel<6, long long><<<(int)blocks, 256, 0, s>>>(a); break;
-        case 8: assemble_kernel<8, long long><<<(int)blocks, 256, 0, s>>>(a); break;
+        case 2: go(assemble_kernel<2, long long>); break;
+        case 4: go(assemble_kernel<4, long long>); break;
+        case 6: go(assemble_kernel<6, long long>); break;
+        case 8: go(assemble_kernel<8, long long>); break;
         default: break;
     }
 }

@@ -19,6 +19,30 @@ namespace ccqb {
 // message returned by ccq_b200_last_error() on this thread
 void set_last_error(const char *msg);
 
+// Programmatic dependent launch.  A kernel launched with launch_after may start while the kernel before it on the same
+// stream is still running; everything it reads or writes that another kernel touches comes after gdc_wait, which
+// every thread of it executes.  gdc_launch lets the next such kernel start.  A sweep of a small system is a chain of
+// about 25 dependent launches; starting each one (its item and tables loaded) before the last has drained took six
+// iterations of CCSD at 8 orbitals from 0.95 to 0.86 ms, at 20 from 1.23 to 1.14, CCSDT at 13 from 1.74 to 1.61.
+__device__ __forceinline__ void gdc_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void gdc_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline void launch_after(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+// Grids above this start only when the kernel before has ended: waiting blocks would hold the SMs against other streams.
+constexpr long long kEarlyBlocks = 148 * 2;
+
 constexpr int MAXR = 8;        // max tensor rank (T4 blocks)
 constexpr int MAX_TERMS = 65536; // max views gathered by one assemble
 

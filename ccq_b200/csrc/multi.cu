@@ -102,6 +102,7 @@ __device__ __forceinline__ void multi_tile(const MultiItem &it, double *red, int
         for (int j = 0; j < NI; ++j)
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0;
+    gdc_wait();   // the tables above are constant; operands and output may be the previous kernel's
     __syncthreads();
     if (wm < it.m) {
         const int step = ks ? 4 : 1;
@@ -204,6 +205,7 @@ constexpr int RED = 4 * 32 * 18;
 __global__ void __launch_bounds__(MT_THREADS, 7) gett_multi_kernel(const MultiItem *__restrict__ items) {
     __shared__ __align__(16) double sm[RED];
     __shared__ int sa[MULTI_K], sb[MULTI_K];
+    gdc_launch();
     const MultiItem it = items[blockIdx.x];
     switch (it.flags >> MI_SHAPE) {
         case 0: multi_tile<1, 2>(it, sm, sa, sb); break;
@@ -212,6 +214,7 @@ __global__ void __launch_bounds__(MT_THREADS, 7) gett_multi_kernel(const MultiIt
         case 3: multi_tile<1, 4>(it, sm, sa, sb); break;
         case MS_VEC: {
             // one column, a few k: one thread per row, no tile
+            gdc_wait();
             for (int m = threadIdx.x; m < it.m; m += MT_THREADS) {
                 const long long ra = __ldg(it.am + m), rb = __ldg(it.bn);
                 double v = 0.0;
@@ -223,6 +226,7 @@ __global__ void __launch_bounds__(MT_THREADS, 7) gett_multi_kernel(const MultiIt
         }
         default: {
             // copy (A to C) or zero (A null) of m values
+            gdc_wait();
             for (int i = threadIdx.x; i < it.m; i += MT_THREADS) it.C[i] = it.A ? __ldg(it.A + i) : 0.0;
         }
     }
@@ -230,7 +234,9 @@ __global__ void __launch_bounds__(MT_THREADS, 7) gett_multi_kernel(const MultiIt
 
 __global__ void __launch_bounds__(MT_THREADS, 4) gett_multi64_kernel(const MultiItem *__restrict__ items) {
     __shared__ __align__(16) double sm[4 * TILE];   // two stages of both operands
+    gdc_launch();
     const MultiItem it = items[blockIdx.x];
+    gdc_wait();
     switch ((it.flags >> MI_SHAPE) - MS_64) {
         case 0: multi_tile64<false, false>(it, sm); break;
         case 1: multi_tile64<false, true>(it, sm); break;
@@ -244,9 +250,9 @@ __global__ void __launch_bounds__(MT_THREADS, 4) gett_multi64_kernel(const Multi
 void launch_gett_multi(const MultiItem *items, int n, bool tiles64, cudaStream_t s) {
     if (n <= 0) return;
     if (tiles64)
-        gett_multi64_kernel<<<n, MT_THREADS, 0, s>>>(items);
+        launch_after(n <= kEarlyBlocks, gett_multi64_kernel, n, MT_THREADS, 0, s, items);
     else
-        gett_multi_kernel<<<n, MT_THREADS, 0, s>>>(items);
+        launch_after(n <= kEarlyBlocks, gett_multi_kernel, n, MT_THREADS, 0, s, items);
 }
 
 cudaError_t preload_multi() {
