@@ -1002,6 +1002,68 @@ __device__ __forceinline__ void canonical_element(const AsmArgs &a, Off lin, int
     }
 }
 
+// Term descriptors [t0, t0 + nt) of an assemble into shared memory.
+template <int RK>
+__device__ __forceinline__ void stage_terms(const AsmArgs &a, SmTerm<RK> *st, int t0, int nt) {
+    for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+        const AsmTerm &g = a.terms[t0 + t];
+        SmTerm<RK> q;
+        q.p = g.p;
+        q.coef = g.coef;
+        unsigned long long pm = 0;
+        for (int gi = 0; gi < g.ng; ++gi)
+            for (int u = 0; u < g.glen[gi]; ++u)
+                for (int v = u + 1; v < g.glen[gi]; ++v) {
+                    int j = g.gpos[gi][u], k = g.gpos[gi][v];
+                    if (j > k) {
+                        int tmp = j;
+                        j = k;
+                        k = tmp;
+                    }
+                    pm |= 1ull << (j * RK + k);
+                }
+        q.pm = pm;
+#pragma unroll
+        for (int d = 0; d < RK; ++d) {
+            q.zs[d] = g.zstride[d];
+            q.src[d] = (unsigned char)g.src[d];
+            q.tst[d] = 0;
+        }
+#pragma unroll
+        for (int j = 0; j < RK; ++j) q.tst[g.src[j]] += g.zstride[j];
+        st[t] = q;
+    }
+}
+
+// The term's value at element x, a view read sorted with sign.
+template <int RK, typename Off>
+__device__ __forceinline__ double sorted_term(const SmTerm<RK> &q, const int (&x)[RK]) {
+    double sg = q.coef;
+    int y[RK];
+#pragma unroll
+    for (int j = 0; j < RK; ++j) y[j] = pick<RK>(x, q.src[j]);
+    // selection sort within groups: one sign flip per exchange
+#pragma unroll
+    for (int j = 0; j < RK; ++j)
+#pragma unroll
+        for (int k = j + 1; k < RK; ++k)
+            if ((q.pm >> (j * RK + k)) & 1ull) {
+                if (y[j] > y[k]) {
+                    const int tmp = y[j];
+                    y[j] = y[k];
+                    y[k] = tmp;
+                    sg = -sg;
+                } else if (y[j] == y[k]) {
+                    sg = 0.0;
+                }
+            }
+    if (sg == 0.0) return 0.0;
+    Off off = 0;
+#pragma unroll
+    for (int j = 0; j < RK; ++j) off += (Off)q.zs[j] * y[j];
+    return sg * __ldg(q.p + off);
+}
+
 // Off: index type of every offset (int when AsmArgs::off32 says they all fit)
 // The canonical elements [base0, total) of one assemble, blockDim.x * ASM_EPT of them per step.
 constexpr int ASM_PMAX = 64;   // orbit permutations whose write strides are staged in shared memory
@@ -1052,34 +1114,7 @@ __device__ __forceinline__ void assemble_body(const AsmArgs &a, SmTerm<RK> (&st)
         for (int c = 0; c < nch; ++c) {
             __syncthreads();
             const int nt = min(CH, a.nterms - c * CH);
-            for (int t = threadIdx.x; t < nt; t += blockDim.x) {
-                const AsmTerm &g = a.terms[c * CH + t];
-                SmTerm<RK> q;
-                q.p = g.p;
-                q.coef = g.coef;
-                unsigned long long pm = 0;
-                for (int gi = 0; gi < g.ng; ++gi)
-                    for (int u = 0; u < g.glen[gi]; ++u)
-                        for (int v = u + 1; v < g.glen[gi]; ++v) {
-                            int j = g.gpos[gi][u], k = g.gpos[gi][v];
-                            if (j > k) {
-                                int tmp = j;
-                                j = k;
-                                k = tmp;
-                            }
-                            pm |= 1ull << (j * RK + k);
-                        }
-                q.pm = pm;
-#pragma unroll
-                for (int d = 0; d < RK; ++d) {
-                    q.zs[d] = g.zstride[d];
-                    q.src[d] = (unsigned char)g.src[d];
-                    q.tst[d] = 0;
-                }
-#pragma unroll
-                for (int j = 0; j < RK; ++j) q.tst[g.src[j]] += g.zstride[j];
-                st[t] = q;
-            }
+            stage_terms<RK>(a, st, c * CH, nt);
             __syncthreads();
             // plain views first (a branch-free loop, so the loads of several terms are in flight
             // together), then the views read sorted with sign
@@ -1101,39 +1136,9 @@ __device__ __forceinline__ void assemble_body(const AsmArgs &a, SmTerm<RK> (&st)
             }
 #pragma unroll 2
             for (int t = np; t < nt; ++t) {
-                const SmTerm<RK> &q = st[t];
-                const double *p = q.p;
-                {
 #pragma unroll
-                    for (int e = 0; e < ASM_EPT; ++e) {
-                        if (!need[e]) continue;
-                        double sg = q.coef;
-                        int y[RK];
-#pragma unroll
-                        for (int j = 0; j < RK; ++j) y[j] = pick<RK>(x[e], q.src[j]);
-                        bool zero = false;
-                        // selection sort within groups: one sign flip per exchange
-#pragma unroll
-                        for (int j = 0; j < RK; ++j)
-#pragma unroll
-                            for (int k = j + 1; k < RK; ++k)
-                                if ((q.pm >> (j * RK + k)) & 1ull) {
-                                    if (y[j] > y[k]) {
-                                        int tmp = y[j];
-                                        y[j] = y[k];
-                                        y[k] = tmp;
-                                        sg = -sg;
-                                    } else if (y[j] == y[k]) {
-                                        zero = true;
-                                    }
-                                }
-                        if (zero) continue;
-                        Off off = 0;
-#pragma unroll
-                        for (int j = 0; j < RK; ++j) off += (Off)q.zs[j] * y[j];
-                        R[e] += sg * __ldg(p + off);
-                    }
-                }
+                for (int e = 0; e < ASM_EPT; ++e)
+                    if (need[e]) R[e] += sorted_term<RK, Off>(st[t], x[e]);
             }
         }
 #pragma unroll
@@ -1196,6 +1201,101 @@ __global__ void __launch_bounds__(256, 4) assemble_kernel(AsmArgs a) {
                                (long long)gridDim.x * blockDim.x * ASM_EPT);
 }
 
+// Few canonical elements, many terms or images (the T4 blocks of small systems: 210 elements, 826 terms, 576
+// images): G neighbouring lanes share an element, taking its terms and then its images in turn.  With a thread per
+// element such a block is one serial chain of loads and scattered stores on a few SMs (T4A of 14 orbitals 373 us, its
+// copy T4E 203 us, T3A of 24 orbitals 41 us of an eager sweep).  A pass of six iterations: CCSDT 13 orbitals 1.60 -> 1.48
+// ms, 24 orbitals 6.65 -> 6.53 ms, CCSDTQ 14 orbitals 45.2 -> 42.9 ms.
+template <int RK, typename Off, int G>
+__global__ void __launch_bounds__(256) assemble_group_kernel(AsmArgs a) {
+    constexpr int CH = 128;
+    __shared__ SmTerm<RK> st[CH];
+    gdc_launch();
+    gdc_wait();
+    const int lane = threadIdx.x % G;
+    const long long lin = blockIdx.x * (long long)(blockDim.x / G) + threadIdx.x / G;
+    const bool act = lin < a.total;
+    int x[RK];
+#pragma unroll
+    for (int d = 0; d < RK; ++d) x[d] = 0;
+    if (act) canonical_element<RK, Off>(a, (Off)lin, x);
+    bool need = act;
+    if (a.act && act) {
+        // CCSDt: at least one active occupied and one active virtual index
+        bool occ = false, vir = false;
+#pragma unroll
+        for (int d = 0; d < RK; ++d) {
+            if (d < RK / 2)
+                occ = occ || x[d] >= a.act_occ_lo;
+            else
+                vir = vir || x[d] < a.act_vir_hi[a.spin[d]];
+        }
+        need = occ && vir;
+    }
+    double R = 0.0;
+    for (int t0 = 0; t0 < a.nterms; t0 += CH) {
+        __syncthreads();
+        const int nt = min(CH, a.nterms - t0);
+        stage_terms<RK>(a, st, t0, nt);
+        __syncthreads();
+        if (!need) continue;
+        const int np = min(max(a.nplain - t0, 0), nt);
+#pragma unroll 4
+        for (int t = lane; t < np; t += G) {
+            Off off = 0;
+#pragma unroll
+            for (int d = 0; d < RK; ++d) off += (Off)st[t].tst[d] * x[d];
+            R += st[t].coef * __ldg(st[t].p + off);
+        }
+#pragma unroll 2
+        for (int t = np + lane; t < nt; t += G) R += sorted_term<RK, Off>(st[t], x);
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) R += __shfl_xor_sync(0xffffffffu, R, o);
+    Off toff = 0;
+#pragma unroll
+    for (int d = 0; d < RK; ++d) toff += (Off)a.tstride[d] * x[d];
+    const double told = act && a.mode != 1 ? a.T[toff] : 0.0;
+    __syncwarp();   // every lane of the group has read T before an image overwrites it
+    if (act) {
+        double tnew = R;
+        if (a.mode != 1) {
+            double D = a.shift;
+            if (a.mode == 2) D -= *a.ecor;
+#pragma unroll
+            for (int d = 0; d < RK; ++d) {
+                if (d < RK / 2)
+                    D -= a.fdiag[a.spin[d]][x[d]];
+                else
+                    D += a.fdiag[a.spin[d]][a.nocc[a.spin[d]] + x[d]];
+            }
+            tnew = told - R / D;
+            if (!need) tnew = 0.0;   // triples outside the active space stay zero
+        }
+        for (int pidx = lane; pidx < a.nperm; pidx += G) {
+            const signed char *P = a.perm + pidx * RK;
+            Off o = 0;
+#pragma unroll
+            for (int d = 0; d < RK; ++d) o += (Off)a.tstride[d] * pick<RK>(x, __ldg(P + d));
+            a.T[o] = a.psign[pidx] * tnew;
+        }
+    }
+    if (a.mode == 2) {
+        double nacc = (act && lane == 0) ? a.nperm * R * R : 0.0;
+        for (int o = 16; o > 0; o >>= 1) nacc += __shfl_down_sync(0xffffffffu, nacc, o);
+        if ((threadIdx.x & 31) == 0 && nacc != 0.0) atomicAdd(a.norm, nacc);
+    }
+}
+
+// Lanes per element of an assemble: enough that the elements fill the chip's threads once (148 SMs of 2048), where an
+// element has that much to share.
+int assemble_lanes(const AsmArgs &a) {
+    const int work = a.nterms + a.nperm;
+    if (a.total * 32 <= 148 * 2048 && work >= 64) return 32;
+    if (a.total * 8 <= 148 * 2048 && work >= 16) return 8;
+    return 1;
+}
+
 // Many assembles of the same rank in one launch (one per context of a batch of independent
 // solves): block b handles the chunk b - cstart[i] (256 * ASM_EPT canonical elements) of assemble
 // i, where cstart[i] <= b < cstart[i + 1]; assemble i is skipped when active[owner[i]] is zero.
@@ -1253,6 +1353,18 @@ void launch_copy_batched(const BatchCopy *cp, int n, const int *owner, const int
 }
 
 void launch_assemble(const AsmArgs &a, cudaStream_t s) {
+    if (const int g = a.off32 ? assemble_lanes(a) : 1; g > 1 && a.total > 0) {
+        const long long nb = (a.total * g + 255) / 256;
+        auto go = [&](auto kernel) { launch_after(nb <= kEarlyBlocks, kernel, (unsigned)nb, 256, 0, s, a); };
+        switch (a.rank) {
+            case 2: go(g == 8 ? assemble_group_kernel<2, int, 8> : assemble_group_kernel<2, int, 32>); break;
+            case 4: go(g == 8 ? assemble_group_kernel<4, int, 8> : assemble_group_kernel<4, int, 32>); break;
+            case 6: go(g == 8 ? assemble_group_kernel<6, int, 8> : assemble_group_kernel<6, int, 32>); break;
+            case 8: go(g == 8 ? assemble_group_kernel<8, int, 8> : assemble_group_kernel<8, int, 32>); break;
+            default: break;
+        }
+        return;
+    }
     long long blocks = (a.total + 256 * ASM_EPT - 1) / (256 * ASM_EPT);
     if (blocks > 148 * 32) blocks = 148 * 32;
     if (blocks < 1) blocks = 1;
@@ -1551,6 +1663,14 @@ cudaError_t preload_kernels(int ds) {
     touch((const void *)fill_kernel);
     touch((const void *)ring_step_kernel);
     touch((const void *)diis_extrap_kernel);
+    touch((const void *)assemble_group_kernel<2, int, 8>);
+    touch((const void *)assemble_group_kernel<4, int, 8>);
+    touch((const void *)assemble_group_kernel<6, int, 8>);
+    touch((const void *)assemble_group_kernel<8, int, 8>);
+    touch((const void *)assemble_group_kernel<2, int, 32>);
+    touch((const void *)assemble_group_kernel<4, int, 32>);
+    touch((const void *)assemble_group_kernel<6, int, 32>);
+    touch((const void *)assemble_group_kernel<8, int, 32>);
     touch((const void *)assemble_kernel<2, int>);
     touch((const void *)assemble_kernel<4, int>);
     touch((const void *)assemble_kernel<6, int>);

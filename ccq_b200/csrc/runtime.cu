@@ -2242,8 +2242,8 @@ void run_node(ccq_b200_ctx *c, const Sched &s, const SchedNode &n, cudaStream_t 
     }
 }
 
-// The launches of plan operations [from, to) issued on the context's stream one after the other, or (dag, under
-// capture) on side streams with the dependencies as edges, so that independent launches run at the same time.
+// The launches of plan operations [from, to) issued on the context's stream one after the other, or (dag) on side
+// streams with the dependencies as event waits (edges, under capture), so that independent launches run at the same time.
 void run_sched(ccq_b200_ctx *c, size_t from, size_t to, bool dag) {
     const Sched &s = sched_for(c, from, to);
     auto out_after = [&](const SchedNode &n, cudaStream_t st) {
@@ -2352,11 +2352,12 @@ void run_sched(ccq_b200_ctx *c, size_t from, size_t to, bool dag) {
 
 void run_ops(ccq_b200_ctx *c, size_t from, size_t to);
 
-// A range that is run once per solve (not captured): scheduled on the context's stream, or operation by
+// A range that is run once per solve (not captured): scheduled over the side streams (left preparation, six left
+// iterations and corrections at 32 orbitals 13.0 -> 11.8 ms against the context's stream alone), or operation by
 // operation while profiling and with graphs off.
 void run_range(ccq_b200_ctx *c, size_t from, size_t to) {
     if (c->use_graph && !c->profile)
-        run_sched(c, from, to, false);
+        run_sched(c, from, to, true);
     else
         run_ops(c, from, to);
 }
