@@ -109,3 +109,21 @@ def test_diis_space(ds):
     np.testing.assert_allclose([g[0] for g in got], [x[0] for x in hist], atol=1e-11, rtol=0)
     np.testing.assert_allclose([g[1] ** 2 for g in got], [x[2] ** 2 for x in hist], atol=1e-11, rtol=0)
     ctx.close()
+
+
+def test_large_pageable_blocks_round_trip():
+    """Blocks on both sides of the size that is copied by several threads, of odd lengths, and the whole vector."""
+    ctx, d = _context('CCSDTQ', 12, 4, 3, 0)
+    shapes = _shapes(d, ('T4A', 'T4B', 'T4C', 'T4D', 'T3B', 'T2B'))
+    sizes = [8 * int(np.prod(s)) for s in shapes.values()]
+    assert max(sizes) >= 2 * (4 << 20) and min(sizes) < 4 << 20
+    rng = np.random.default_rng(3)
+    put = {b: rng.normal(size=s) for b, s in shapes.items()}
+    for b, x in put.items():
+        ctx.set_block(b, x)
+    for b, x in put.items():
+        assert np.array_equal(ctx.get_block(b, shapes[b]), x), b
+    t = rng.normal(size=ctx.t_size)
+    ctx.set_t(t)
+    assert np.array_equal(ctx.get_t(), t)
+    ctx.close()
