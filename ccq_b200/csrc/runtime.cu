@@ -471,8 +471,13 @@ void ring_and_diis(ccq_b200_ctx *c, double *ring, const double *vec, long long v
 constexpr int kCopyThreads = 4;
 constexpr size_t kCopySlot = 2ull << 20, kCopyMin = 4ull << 20;
 
-void copy_pageable(ccq_b200_ctx *c, char *host, char *dev, size_t bytes, bool to_device) {
-    if (!c->stage) CK(cudaMallocHost((void **)&c->stage, kCopyThreads * 2 * kCopySlot));
+// false: no pinned memory to be had, nothing was copied
+bool copy_pageable(ccq_b200_ctx *c, char *host, char *dev, size_t bytes, bool to_device) {
+    if (!c->stage && cudaMallocHost((void **)&c->stage, kCopyThreads * 2 * kCopySlot) != cudaSuccess) {
+        cudaGetLastError();
+        c->stage = nullptr;
+        return false;
+    }
     while ((int)c->stage_st.size() < kCopyThreads) {
         cudaStream_t st;
         CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
@@ -521,10 +526,17 @@ void copy_pageable(ccq_b200_ctx *c, char *host, char *dev, size_t bytes, bool to
     };
     {
         Join join{th};
-        for (int t = 1; t < kCopyThreads; ++t) th.emplace_back(work, t);
+        int t = 1;
+        try {
+            th.reserve(kCopyThreads);
+            for (; t < kCopyThreads; ++t) th.emplace_back(work, t);
+        } catch (const std::exception &) {
+            for (; t < kCopyThreads; ++t) work(t);   // no more threads: their shares here
+        }
         work(0);
     }
     for (cudaError_t e : err) CK(e);
+    return true;
 }
 
 void copy_user(ccq_b200_ctx *c, double *host, double *dev, long long n, bool to_device) {
@@ -533,10 +545,7 @@ void copy_user(ccq_b200_ctx *c, double *host, double *dev, long long n, bool to_
         cudaPointerAttributes pa{};
         const bool pinned = cudaPointerGetAttributes(&pa, host) == cudaSuccess && pa.type != cudaMemoryTypeUnregistered;
         cudaGetLastError();
-        if (!pinned) {
-            copy_pageable(c, (char *)host, (char *)dev, bytes, to_device);
-            return;
-        }
+        if (!pinned && copy_pageable(c, (char *)host, (char *)dev, bytes, to_device)) return;
     }
     CK(cudaMemcpyAsync(to_device ? (void *)dev : (void *)host, to_device ? (const void *)host : (const void *)dev, bytes,
                        to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, c->stream));
