@@ -10,6 +10,18 @@ __device__ __forceinline__ double at4(const double *p, int a, int b, int c, int 
     return __ldg(p + ((static_cast<long long>(a) * n1 + b) * n2 + c) * n3 + d);
 }
 
+// sum of f(i, j) over i < n1, j < n2 by the lanes of a warp, the same value in all of them
+template <typename F>
+__device__ __forceinline__ double lane_sum(int n1, int n2, F f) {
+    double s = 0.0;
+    const int total = n1 * n2;
+#pragma unroll 4
+    for (int x = threadIdx.x & 31; x < total; x += 32) s += f(x / n2, x % n2);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
 // Hbar one-body diagonal h(p,p) of one spin (sigma = 0 alpha, 1 beta), full-range p:
 //   occupied  h(i,i) = f~(i,i) + 1/2 sum_{m e f} <im||ef> t(ef,im)
 //   virtual   h(a,a) = f~(a,a) - 1/2 sum_{m n f} <mn||af> t(af,mn)
@@ -22,26 +34,26 @@ __device__ double hbar1(const CrDiagArgs &g, int sigma, int p) {
         if (p < oa) {
             const int i = p;
             double x = 0.0, y = 0.0;
-            for (int m = 0; m < oa; ++m)
-                for (int e = 0; e < va; ++e)
-                    for (int f = 0; f < va; ++f)
-                        x += at4(g.VAA0, i, m, oa + e, oa + f, n, n, n) * at4(g.T2A, i, m, e, f, oa, va, va);
-            for (int m = 0; m < ob; ++m)
-                for (int e = 0; e < va; ++e)
-                    for (int f = 0; f < vb; ++f)
-                        y += at4(g.VAB0, i, m, oa + e, ob + f, n, n, n) * at4(g.T2B, i, m, e, f, ob, va, vb);
+            x = lane_sum(oa * va, va, [&](int me, int f) {
+                const int m = me / va, e = me % va;
+                return at4(g.VAA0, i, m, oa + e, oa + f, n, n, n) * at4(g.T2A, i, m, e, f, oa, va, va);
+            });
+            y = lane_sum(ob * va, vb, [&](int me, int f) {
+                const int m = me / va, e = me % va;
+                return at4(g.VAB0, i, m, oa + e, ob + f, n, n, n) * at4(g.T2B, i, m, e, f, ob, va, vb);
+            });
             s += 0.5 * x + y;
         } else {
             const int a = p - oa;
             double x = 0.0, y = 0.0;
-            for (int m = 0; m < oa; ++m)
-                for (int q = 0; q < oa; ++q)
-                    for (int f = 0; f < va; ++f)
-                        x += at4(g.VAA0, m, q, p, oa + f, n, n, n) * at4(g.T2A, m, q, a, f, oa, va, va);
-            for (int m = 0; m < oa; ++m)
-                for (int q = 0; q < ob; ++q)
-                    for (int f = 0; f < vb; ++f)
-                        y += at4(g.VAB0, m, q, p, ob + f, n, n, n) * at4(g.T2B, m, q, a, f, ob, va, vb);
+            x = lane_sum(oa * oa, va, [&](int mq, int f) {
+                const int m = mq / oa, q = mq % oa;
+                return at4(g.VAA0, m, q, p, oa + f, n, n, n) * at4(g.T2A, m, q, a, f, oa, va, va);
+            });
+            y = lane_sum(oa * ob, vb, [&](int mq, int f) {
+                const int m = mq / ob, q = mq % ob;
+                return at4(g.VAB0, m, q, p, ob + f, n, n, n) * at4(g.T2B, m, q, a, f, ob, va, vb);
+            });
             s -= 0.5 * x + y;
         }
     } else {
@@ -49,26 +61,26 @@ __device__ double hbar1(const CrDiagArgs &g, int sigma, int p) {
         if (p < ob) {
             const int i = p;
             double x = 0.0, y = 0.0;
-            for (int m = 0; m < ob; ++m)
-                for (int e = 0; e < vb; ++e)
-                    for (int f = 0; f < vb; ++f)
-                        x += at4(g.VBB0, i, m, ob + e, ob + f, n, n, n) * at4(g.T2C, i, m, e, f, ob, vb, vb);
-            for (int m = 0; m < oa; ++m)
-                for (int e = 0; e < va; ++e)
-                    for (int f = 0; f < vb; ++f)
-                        y += at4(g.VAB0, m, i, oa + e, ob + f, n, n, n) * at4(g.T2B, m, i, e, f, ob, va, vb);
+            x = lane_sum(ob * vb, vb, [&](int me, int f) {
+                const int m = me / vb, e = me % vb;
+                return at4(g.VBB0, i, m, ob + e, ob + f, n, n, n) * at4(g.T2C, i, m, e, f, ob, vb, vb);
+            });
+            y = lane_sum(oa * va, vb, [&](int me, int f) {
+                const int m = me / va, e = me % va;
+                return at4(g.VAB0, m, i, oa + e, ob + f, n, n, n) * at4(g.T2B, m, i, e, f, ob, va, vb);
+            });
             s += 0.5 * x + y;
         } else {
             const int a = p - ob;
             double x = 0.0, y = 0.0;
-            for (int m = 0; m < ob; ++m)
-                for (int q = 0; q < ob; ++q)
-                    for (int f = 0; f < vb; ++f)
-                        x += at4(g.VBB0, m, q, p, ob + f, n, n, n) * at4(g.T2C, m, q, a, f, ob, vb, vb);
-            for (int m = 0; m < oa; ++m)
-                for (int q = 0; q < ob; ++q)
-                    for (int f = 0; f < va; ++f)
-                        y += at4(g.VAB0, m, q, oa + f, p, n, n, n) * at4(g.T2B, m, q, f, a, ob, va, vb);
+            x = lane_sum(ob * ob, vb, [&](int mq, int f) {
+                const int m = mq / ob, q = mq % ob;
+                return at4(g.VBB0, m, q, p, ob + f, n, n, n) * at4(g.T2C, m, q, a, f, ob, vb, vb);
+            });
+            y = lane_sum(oa * ob, va, [&](int mq, int f) {
+                const int m = mq / ob, q = mq % ob;
+                return at4(g.VAB0, m, q, oa + f, p, n, n, n) * at4(g.T2B, m, q, f, a, ob, va, vb);
+            });
             s -= 0.5 * x + y;
         }
     }
@@ -93,28 +105,31 @@ __device__ double hbar2_same(const CrDiagArgs &g, int sigma, int p, int q) {
     double s = at4(V, p, q, p, q, n, n, n);
     if (p < o && q < o) {
         double x = 0.0;
-        for (int e = 0; e < v; ++e)
-            for (int f = 0; f < v; ++f) x += at4(V0, p, q, o + e, o + f, n, n, n) * at4(T, p, q, e, f, o, v, v);
+        x = lane_sum(v, v, [&](int e, int f) {
+            return at4(V0, p, q, o + e, o + f, n, n, n) * at4(T, p, q, e, f, o, v, v);
+        });
         s += 0.5 * x;
     } else if (p >= o && q >= o) {
         double x = 0.0;
-        for (int m = 0; m < o; ++m)
-            for (int k = 0; k < o; ++k) x += at4(V0, m, k, p, q, n, n, n) * at4(T, m, k, p - o, q - o, o, v, v);
+        x = lane_sum(o, o, [&](int m, int k) {
+            return at4(V0, m, k, p, q, n, n, n) * at4(T, m, k, p - o, q - o, o, v, v);
+        });
         s += 0.5 * x;
     } else {
         // p virtual (a), q occupied (i)
         const int a = p - o, i = q;
         double x = 0.0, y = 0.0;
-        for (int k = 0; k < o; ++k)
-            for (int f = 0; f < v; ++f) x += at4(V0, i, k, p, o + f, n, n, n) * at4(T, i, k, a, f, o, v, v);
+        x = lane_sum(o, v, [&](int k, int f) {
+            return at4(V0, i, k, p, o + f, n, n, n) * at4(T, i, k, a, f, o, v, v);
+        });
         if (sigma == 0) {
-            for (int k = 0; k < g.ob; ++k)
-                for (int f = 0; f < g.vb; ++f)
-                    y += at4(g.VAB0, i, k, p, g.ob + f, n, n, n) * at4(g.T2B, i, k, a, f, g.ob, g.va, g.vb);
+            y = lane_sum(g.ob, g.vb, [&](int k, int f) {
+                return at4(g.VAB0, i, k, p, g.ob + f, n, n, n) * at4(g.T2B, i, k, a, f, g.ob, g.va, g.vb);
+            });
         } else {
-            for (int k = 0; k < g.oa; ++k)
-                for (int f = 0; f < g.va; ++f)
-                    y += at4(g.VAB0, k, i, g.oa + f, p, n, n, n) * at4(g.T2B, k, i, f, a, g.ob, g.va, g.vb);
+            y = lane_sum(g.oa, g.va, [&](int k, int f) {
+                return at4(g.VAB0, k, i, g.oa + f, p, n, n, n) * at4(g.T2B, k, i, f, a, g.ob, g.va, g.vb);
+            });
         }
         s -= x + y;
     }
@@ -127,26 +142,26 @@ __device__ double hbar2_ab(const CrDiagArgs &g, int p, int q) {
     double s = at4(g.VAB, p, q, p, q, n, n, n);
     double x = 0.0;
     if (p < oa && q < ob) {
-        for (int e = 0; e < va; ++e)
-            for (int f = 0; f < vb; ++f)
-                x += at4(g.VAB0, p, q, oa + e, ob + f, n, n, n) * at4(g.T2B, p, q, e, f, ob, va, vb);
+        x = lane_sum(va, vb, [&](int e, int f) {
+            return at4(g.VAB0, p, q, oa + e, ob + f, n, n, n) * at4(g.T2B, p, q, e, f, ob, va, vb);
+        });
         s += x;
     } else if (p >= oa && q >= ob) {
-        for (int m = 0; m < oa; ++m)
-            for (int k = 0; k < ob; ++k)
-                x += at4(g.VAB0, m, k, p, q, n, n, n) * at4(g.T2B, m, k, p - oa, q - ob, ob, va, vb);
+        x = lane_sum(oa, ob, [&](int m, int k) {
+            return at4(g.VAB0, m, k, p, q, n, n, n) * at4(g.T2B, m, k, p - oa, q - ob, ob, va, vb);
+        });
         s += x;
     } else if (p >= oa) {
         // alpha virtual a = p, beta occupied i = q
-        for (int k = 0; k < oa; ++k)
-            for (int f = 0; f < vb; ++f)
-                x += at4(g.VAB0, k, q, p, ob + f, n, n, n) * at4(g.T2B, k, q, p - oa, f, ob, va, vb);
+        x = lane_sum(oa, vb, [&](int k, int f) {
+            return at4(g.VAB0, k, q, p, ob + f, n, n, n) * at4(g.T2B, k, q, p - oa, f, ob, va, vb);
+        });
         s -= x;
     } else {
         // alpha occupied i = p, beta virtual a = q
-        for (int k = 0; k < ob; ++k)
-            for (int f = 0; f < va; ++f)
-                x += at4(g.VAB0, p, k, oa + f, q, n, n, n) * at4(g.T2B, p, k, f, q - ob, ob, va, vb);
+        x = lane_sum(ob, va, [&](int k, int f) {
+            return at4(g.VAB0, p, k, oa + f, q, n, n, n) * at4(g.T2B, p, k, f, q - ob, ob, va, vb);
+        });
         s -= x;
     }
     return s;
@@ -215,33 +230,33 @@ __device__ double w2(const CrDiagArgs &g, int c, int x, int z, int y) {
     }
 }
 
+// The one- and two-body diagonals sum over up to o v^2 pairs each: a warp per value (a thread per value was one serial
+// chain of loads, 0.67 ms at 32 orbitals).  The three-body ones sum over one index: a thread per value.
 __global__ void crdiag_kernel(CrDiagArgs g) {
     const long long n = g.n, n2 = n * n, n3 = n2 * n;
-    const long long total = 2 * n + 3 * n2 + 8 * n3;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        long long r = t;
-        if (r < 2 * n) {
-            const int sigma = (int)(r / n), p = (int)(r % n);
-            (sigma ? g.HDB : g.HDA)[p] = hbar1(g, sigma, p);
+    const long long thread = blockIdx.x * (long long)blockDim.x + threadIdx.x, threads = (long long)gridDim.x * blockDim.x;
+    const bool first = (threadIdx.x & 31) == 0;
+    for (long long t = thread >> 5; t < 2 * n + 3 * n2; t += threads >> 5) {
+        if (t < 2 * n) {
+            const int sigma = (int)(t / n), p = (int)(t % n);
+            const double v = hbar1(g, sigma, p);
+            if (first) (sigma ? g.HDB : g.HDA)[p] = v;
             continue;
         }
-        r -= 2 * n;
-        if (r < 3 * n2) {
-            const int w = (int)(r / n2);
-            const int p = (int)((r % n2) / n), q = (int)(r % n);
-            double v = 0.0;
-            if (w == 1) {
-                v = hbar2_ab(g, p, q);
-            } else if (p != q) {
-                v = hbar2_same(g, w == 0 ? 0 : 1, p, q);
-            }
-            (w == 0 ? g.H2AA : (w == 1 ? g.H2AB : g.H2BB))[r % n2] = v;
-            continue;
+        const long long r = t - 2 * n;
+        const int w = (int)(r / n2);
+        const int p = (int)((r % n2) / n), q = (int)(r % n);
+        double v = 0.0;
+        if (w == 1) {
+            v = hbar2_ab(g, p, q);
+        } else if (p != q) {
+            v = hbar2_same(g, w == 0 ? 0 : 1, p, q);
         }
-        r -= 3 * n2;
-        const int w = (int)(r / n3);
-        const long long e = r % n3;
+        if (first) (w == 0 ? g.H2AA : (w == 1 ? g.H2AB : g.H2BB))[r % n2] = v;
+    }
+    for (long long t = thread; t < 8 * n3; t += threads) {
+        const int w = (int)(t / n3);
+        const long long e = t % n3;
         const int i0 = (int)(e / n2), i1 = (int)((e / n) % n), i2 = (int)(e % n);
         if (w < 4)
             g.W1[w][e] = w1(g, w, i0, i1, i2);
