@@ -856,8 +856,11 @@ void gett_extents(const ccq_b200_ctx *c, const Op &o, long long (&mnk)[3]) {
 // small enough to be added into.  Of 120 / 300 / 400 MFLOP the higher limits are better where many contractions
 // of a few hundred MFLOP wait for each other (CCSDt at 32 orbitals 22.4 / 21.5 / 21.0 ms a pass, the left solve at 32
 // 15.7 / 13.2 / 13.1 ms) and cost 1-2 % at 24 orbitals (7.1 / 7.2 ms); a 40-orbital CCSDT sweep does not see them.
+// Outputs of up to 300 000 / 786 432 / 1 M elements: CCSDT at 24 orbitals, whose largest intermediates have 857 375,
+// 6.02 / 6.01 / 6.51 ms (zeroing and adding cost such an output more than its launch), eight CCSD systems at once
+// 6.05 / 5.43 / 5.40 ms.
 constexpr double kSmallFlops = 400e6;
-constexpr long long kSmallOut = 1 << 20;
+constexpr long long kSmallOut = 3 << 18;
 bool small_gett(const long long (&mnk)[3]) {
     return 2.0 * mnk[0] * mnk[1] * mnk[2] <= kSmallFlops && mnk[0] * mnk[1] <= kSmallOut;
 }
