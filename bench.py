@@ -454,8 +454,8 @@ def batch_leg(rank, world):
             # iterations overlap the context creation: only the wall from start to the last solve means anything
             legs[name]['solves_per_s'] = None
             legs[name]['solve_wall_s'] = None
-    # headline: one captured graph per instance on its own stream (the faster of the two here: the
-    # batched CCSD sweep is bound by the T1 re-dressing of every instance's n^4 integrals, not by launches);
+    # headline: one captured graph per instance on its own stream (the faster of the two: an instance's graph holds
+    # shared launches and the two-pass T1 dressing, the grouped iteration one launch per plan operation);
     # end to end, the pipelined run (instances iterate while the other contexts are being created)
     head = legs['streams']
     solve_s, setup_s = head['solve_wall_s'], head['setup_wall_s']
