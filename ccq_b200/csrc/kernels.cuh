@@ -41,6 +41,7 @@ inline void launch_after(bool early, void (*kernel)(P...), dim3 grid, dim3 block
     cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 // Grids above this start only when the kernel before has ended: waiting blocks would hold the SMs against other streams.
+// (Limit 0 / 296 / 600 / none: CCSD at 8 orbitals 0.97 / 0.86 / 0.86 / 0.86 ms, at 33 1.52 / 1.47 / 1.46 / 1.51.)
 constexpr long long kEarlyBlocks = 148 * 2;
 
 constexpr int MAXR = 8;        // max tensor rank (T4 blocks)

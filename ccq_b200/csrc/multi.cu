@@ -200,8 +200,9 @@ __device__ __forceinline__ void multi_tile64(const MultiItem &it, double *sm) {
 // partial tiles of four warps: 16 x 16, 32 x 8, 32 x 16 or 16 x 32, rows padded by two
 constexpr int RED = 4 * 32 * 18;
 
-// Direct and one-column items, copies: bound by latency, so registers and shared memory are held down to eight
-// blocks per SM instead of loading ahead within a warp.
+// Direct and one-column items, copies: bound by latency, so registers and shared memory are held down to seven
+// blocks per SM instead of loading ahead within a warp (six iterations of CCSDT at 24 orbitals 6.7 ms; with the next
+// slab loaded ahead at 128 registers and four blocks 7.3 ms).
 __global__ void __launch_bounds__(MT_THREADS, 7) gett_multi_kernel(const MultiItem *__restrict__ items) {
     __shared__ __align__(16) double sm[RED];
     __shared__ int sa[MULTI_K], sb[MULTI_K];

@@ -880,7 +880,8 @@ std::vector<size_t> run_ranges(const ccq_b200_ctx *c) {
 // Accumulation buffers: the intermediates that only small contractions write, all before the first read and
 // all in one run range.  They live outside the phases' shared arena, contiguous per range, so that one memset
 // at the range's start zeroes them; their writers then only add, in any order and with any split of K.  At
-// most kZeroBytes per range, smallest first.
+// most kZeroBytes per range, smallest first (the memset runs beside the dressing: 96 MiB take about 30 us, as long as
+// the dressing of a system whose intermediates add up to that).
 constexpr long long kZeroBytes = 96LL << 20;
 std::map<std::string, double *> plan_zeroed(ccq_b200_ctx *c) {
     struct Info {
@@ -1995,9 +1996,12 @@ OpIO op_io(const ccq_b200_ctx *c, const Op &o, bool grouped) {
     return r;
 }
 
-// The items of one contraction term.  64 x 64 tiles when both sides have at least kBigSide rows and the tiles fill
-// the chip; else the longer side goes to the 16-row side of the DMMA, the shorter one to its 8 columns.  K ranges
-// are at most MULTI_K, and half that while the grid is too small to fill the chip.
+// The items of one contraction term.  64 x 64 tiles when both sides have at least kBigSide rows and there are at least
+// kBigTiles tiles of 128 k (a wave of fewer runs 8 slabs behind one another on a few SMs: with a limit of 64 / 128 CCSD
+// at 48 orbitals, 108 tiles for a 351 x 351 x 351 product, took 3.62 / 3.42 ms, CCSDT at 24 orbitals 6.69 / 6.81 ms); else
+// the longer side goes to the 16-row side of the DMMA, the shorter one to its 8 columns.  K ranges are at most MULTI_K, and
+// half that while an operation has at most one item per SM (always half: left solve at 32 orbitals 16.1 against 15.7 ms;
+// always whole: CCSD at 20 orbitals 1.33 against 1.29 ms).
 constexpr long long kBigSide = 48, kBigTiles = 128;
 bool multi_big(const GettArgs &g) {
     return std::min(g.M, g.N) >= kBigSide && g.K > 16 &&
