@@ -2001,7 +2001,8 @@ OpIO op_io(const ccq_b200_ctx *c, const Op &o, bool grouped) {
 // at 48 orbitals, 108 tiles for a 351 x 351 x 351 product, took 3.62 / 3.42 ms, CCSDT at 24 orbitals 6.69 / 6.81 ms); else
 // the longer side goes to the 16-row side of the DMMA, the shorter one to its 8 columns.  K ranges are at most MULTI_K, and
 // half that while an operation has at most one item per SM (always half: left solve at 32 orbitals 16.1 against 15.7 ms;
-// always whole: CCSD at 20 orbitals 1.33 against 1.29 ms).
+// always whole: CCSD at 20 orbitals 1.33 against 1.29 ms).  A term that overwrites its output is one item per tile whatever
+// its K: the items of two K ranges would both store, and one half of the sum would be lost.
 constexpr long long kBigSide = 48, kBigTiles = 128;
 bool multi_big(const GettArgs &g) {
     return std::min(g.M, g.N) >= kBigSide && g.K > 16 &&
@@ -2024,8 +2025,9 @@ void add_items(std::vector<MultiItem> &out, const Op &o, const GettSeg &sg, bool
     multi_shape(shape, rows, cols);
     if (shape < MS_64 && !ks) rows *= 4;
     const long long tm = (M + rows - 1) / rows, tn = (N + cols - 1) / cols;
-    long long kc = tm * tn * ((K + MULTI_K / 2 - 1) / (MULTI_K / 2)) <= 148 ? MULTI_K / 2 : MULTI_K;
+    long long kc = add && tm * tn * ((K + MULTI_K / 2 - 1) / (MULTI_K / 2)) <= 148 ? MULTI_K / 2 : MULTI_K;
     const long long nk = std::max(1LL, (K + kc - 1) / kc);
+    if (!add && nk > 1) throw Error(CCQ_B200_EPLAN, "overwriting contraction in several K ranges");
     kc = ((K + nk - 1) / nk + 15) / 16 * 16;
     for (long long i = 0; i < tm; ++i)
         for (long long j = 0; j < tn; ++j)
@@ -2106,7 +2108,7 @@ Sched build_sched(ccq_b200_ctx *c, size_t from, size_t to) {
             if (!zeroed && o.skip) continue;
             if (o.g.K == 0 && (zeroed || o.g.beta)) continue;
             u.add = zeroed || o.g.beta;
-            // a term that overwrites runs as one item per tile, so its K range is limited
+            // a term that overwrites is one item per tile (add_items), so its K is limited to an item's range
             u.merge = !c->forced && o.small && o.g.K > 0 && !use_split(c, o) &&
                       (u.add || (o.group_ops.empty() && o.g.K <= MULTI_K));
             if (!zeroed && !u.merge) u.add = false;

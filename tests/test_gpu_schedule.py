@@ -127,3 +127,60 @@ def test_large_pageable_blocks_round_trip():
     ctx.set_t(t)
     assert np.array_equal(ctx.get_t(), t)
     ctx.close()
+
+
+# Systems whose intermediates outgrow the accumulation buffers, so that contractions of 128 < K <= 256 which overwrite
+# their output share launches: one item per tile (two K ranges would both store and lose half of the sum, an error
+# of the order of the block itself).  Tolerance: per block, 1e-12 of its largest amplitude; sums of up to 1e5 terms
+# rounded in another order differ by about sqrt(1e5) * 1.1e-16 = 4e-14 of the terms' root sum of squares, which leaves
+# room for a cancellation of 30 and two iterations.
+def _assert_same(ref, others):
+    for hist, t in others:
+        np.testing.assert_allclose(hist, ref[0], rtol=1e-11)
+        for b in t:
+            scale = np.abs(ref[1][b]).max()
+            assert np.isfinite(scale) and scale > 0, b
+            np.testing.assert_allclose(t[b], ref[1][b], atol=1e-12 * scale, rtol=0, err_msg=b)
+
+
+@pytest.mark.parametrize('method,norb,occ_a,occ_b,froz,active', [
+    ('CCSDt', 20, 5, 5, 0, (4, 7)),
+    ('CCSDt', 20, 5, 5, 0, (3, 8)),
+    ('CCSDT', 21, 6, 5, 0, None),
+    ('CCSDT', 19, 7, 6, 0, None),
+    ('CCSDT', 22, 7, 6, 1, None),
+    ('CCSDTQ', 15, 5, 5, 0, None),
+])
+def test_overwriting_contractions(method, norb, occ_a, occ_b, froz, active):
+    ctx, d = _context(method, norb, occ_a, occ_b, froz, active=active)
+    names = T12 + ('T3A', 'T3B', 'T3C', 'T3D') + (('T4A', 'T4B', 'T4C', 'T4D', 'T4E') if method == 'CCSDTQ' else ())
+    ref, *others = _modes(ctx, names, _shapes(d, names))
+    _assert_same(ref, others)
+    ctx.close()
+
+
+@pytest.mark.parametrize('norb,occ_a,occ_b,rhf', [(9, 4, 3, False), (38, 7, 7, True), (33, 12, 11, False)])
+def test_left_ranges(norb, occ_a, occ_b, rhf):
+    """Left preparation, iterations and triples corrections of CR-CC(2,3) in the three modes; the corrections to 1e-11
+    (products of two compared quantities, up to 3e7 of them summed)."""
+    ctx, d = _context('CR-CC(2,3)', norb, occ_a, occ_b, 0, rhf)
+    shapes = _shapes(d, T12)
+    res = []
+    for mode in (0, 1, 2):
+        ctx.use_graph(mode)
+        for b in T12:
+            ctx.set_block(b, np.zeros(shapes[b]))
+        e = [ctx.iterate(it)[0] for it in (1, 2)]
+        if mode:   # the same T as the operations' own, so that what is compared is the left part
+            for b in T12:
+                ctx.set_block(b, t0[b])
+        t0 = {b: ctx.get_block(b, shapes[b]) for b in T12}
+        ctx.lambda_init(res[0][0][1] if mode else e[1])
+        hist = e + [ctx.lambda_iterate(it)[0] for it in (1, 2)]
+        lam = {b.replace('T', 'L'): ctx.get_block(b.replace('T', 'L'), shapes[b]) for b in T12}
+        res.append((np.array(hist), lam, ctx.crcc23()))
+    _assert_same(res[0][:2], [r[:2] for r in res[1:]])
+    assert np.all(np.abs(res[0][2]) > 0)
+    for r in res[1:]:
+        np.testing.assert_allclose(r[2], res[0][2], rtol=1e-11, atol=0)
+    ctx.close()
