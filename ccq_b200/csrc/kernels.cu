@@ -1061,7 +1061,7 @@ __device__ __forceinline__ double sorted_term(const SmTerm<RK> &q, const int (&x
     Off off = 0;
 #pragma unroll
     for (int j = 0; j < RK; ++j) off += (Off)q.zs[j] * y[j];
-    return sg * __ldg(q.p + off);
+    return sg * q.p[off];
 }
 
 // Off: index type of every offset (int when AsmArgs::off32 says they all fit)
@@ -1129,7 +1129,7 @@ __device__ __forceinline__ void assemble_body(const AsmArgs &a, SmTerm<RK> (&st)
                     Off off = 0;
 #pragma unroll
                     for (int d = 0; d < RK; ++d) off += (Off)q.tst[d] * x[e][d];
-                    v[e] = need[e] ? __ldg(p + off) : 0.0;
+                    v[e] = need[e] ? p[off] : 0.0;
                 }
 #pragma unroll
                 for (int e = 0; e < ASM_EPT; ++e) R[e] += q.coef * v[e];
@@ -1245,7 +1245,7 @@ __global__ void __launch_bounds__(256) assemble_group_kernel(AsmArgs a) {
             Off off = 0;
 #pragma unroll
             for (int d = 0; d < RK; ++d) off += (Off)st[t].tst[d] * x[d];
-            R += st[t].coef * __ldg(st[t].p + off);
+            R += st[t].coef * st[t].p[off];
         }
 #pragma unroll 2
         for (int t = np + lane; t < nt; t += G) R += sorted_term<RK, Off>(st[t], x);

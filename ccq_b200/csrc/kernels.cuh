@@ -21,7 +21,9 @@ void set_last_error(const char *msg);
 
 // Programmatic dependent launch.  A kernel launched with launch_after may start while the kernel before it on the same
 // stream is still running; everything it reads or writes that another kernel touches comes after gdc_wait, which
-// every thread of it executes.  gdc_launch lets the next such kernel start.  A sweep of a small system is a chain of
+// every thread of it executes, and is read with ordinary loads: __ldg promises data that is read-only while the kernel
+// lives (the compiler may move such a load ahead of the wait), which holds for tables and items only.  gdc_launch lets
+// the next such kernel start.  A sweep of a small system is a chain of
 // about 25 dependent launches; starting each one (its item and tables loaded) before the last has drained took six
 // iterations of CCSD at 8 orbitals from 0.95 to 0.86 ms, at 20 from 1.23 to 1.14, CCSDT at 13 from 1.74 to 1.61.
 __device__ __forceinline__ void gdc_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -47,11 +47,11 @@ __device__ __forceinline__ void load_slab(Slab<MI, NI> &f, const MultiItem &it, 
     for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-            f.a[mi][q] = in[q >> 1] ? __ldg(it.A + (long long)ra[mi][q & 1] + ka[q >> 1]) : 0.0;
+            f.a[mi][q] = in[q >> 1] ? it.A[(long long)ra[mi][q & 1] + ka[q >> 1]] : 0.0;
 #pragma unroll
     for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
-        for (int q = 0; q < 2; ++q) f.b[ni][q] = in[q] ? __ldg(it.B + (long long)rb[ni] + kb[q]) : 0.0;
+        for (int q = 0; q < 2; ++q) f.b[ni][q] = in[q] ? it.B[(long long)rb[ni] + kb[q]] : 0.0;
 }
 
 template <int MI, int NI>
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(MT_THREADS, 7) gett_multi_kernel(const MultiIt
                 const long long ra = __ldg(it.am + m), rb = __ldg(it.bn);
                 double v = 0.0;
                 for (int k = 0; k < it.k; ++k)
-                    v += __ldg(it.A + ra + __ldg(it.ak + k)) * __ldg(it.B + rb + __ldg(it.bk + k));
+                    v += it.A[ra + __ldg(it.ak + k)] * it.B[rb + __ldg(it.bk + k)];
                 put(it.C + __ldg(it.cm + m) + __ldg(it.cn), it.alpha * v, it.flags & MI_ADD);
             }
             break;
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(MT_THREADS, 7) gett_multi_kernel(const MultiIt
         default: {
             // copy (A to C) or zero (A null) of m values
             gdc_wait();
-            for (int i = threadIdx.x; i < it.m; i += MT_THREADS) it.C[i] = it.A ? __ldg(it.A + i) : 0.0;
+            for (int i = threadIdx.x; i < it.m; i += MT_THREADS) it.C[i] = it.A ? it.A[i] : 0.0;
         }
     }
 }
