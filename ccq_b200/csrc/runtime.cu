@@ -375,7 +375,9 @@ struct ccq_b200_ctx {
     AsmTerm *cin_terms = nullptr;               // device: one term per such block
     long long cin_h2d = 0;                      // bytes the captured host round trip reads from host_in
     long long io_h2d = 0, io_d2h = 0;           // bytes of the last host round trip
-    // pinned slots and streams of copy_pageable (made at its first use)
+    // pinned slots and streams of copy_pageable (made at its first use); stage_mutex: two threads may read one
+    // context at the same time (get_t takes a const one)
+    std::mutex stage_mutex;
     char *stage = nullptr;
     std::vector<cudaStream_t> stage_st;
     cudaStream_t cstream = nullptr;
@@ -473,6 +475,7 @@ constexpr size_t kCopySlot = 2ull << 20, kCopyMin = 4ull << 20;
 
 // false: no pinned memory to be had, nothing was copied
 bool copy_pageable(ccq_b200_ctx *c, char *host, char *dev, size_t bytes, bool to_device) {
+    std::lock_guard<std::mutex> lock(c->stage_mutex);
     if (!c->stage && cudaMallocHost((void **)&c->stage, kCopyThreads * 2 * kCopySlot) != cudaSuccess) {
         cudaGetLastError();
         c->stage = nullptr;

@@ -6,9 +6,12 @@
 //     every range's schedule: dependencies name earlier launches; the items of a shared launch cover their
 //     contractions' products once; in one shared launch an element is stored once or only added to.  deep: for every
 //     element, two launches of which one stores, or one reads and one writes, are ordered by the dependencies.
+//   copies
+//     two threads read two large pageable blocks of one context at the same time.
 #include "../ccq_b200/csrc/runtime.cu"
 
 #include <sys/mman.h>
+#include <unistd.h>
 
 #include <iostream>
 #include <set>
@@ -17,6 +20,7 @@
 
 // ---- the CUDA runtime on host memory: streams run at once, launches do nothing -----------------------------
 namespace {
+bool slow = false;   // a transfer takes time
 std::mutex mem_mutex;
 std::map<void *, size_t> mem;
 cudaError_t get(void **p, size_t n) {
@@ -63,7 +67,10 @@ cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { return handle(s); }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) {
+    if (slow) usleep(100);
+    return cudaSuccess;
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorNotSupported; }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *) { return cudaErrorNotSupported; }
@@ -322,6 +329,33 @@ struct Context {
     ~Context() { ccq_b200_free(c); }
 };
 
+std::string copies() {
+    Context x("CCSDT", 0, 5, 5, 22, false, -1, -1);
+    const char *name[2] = {"T3A", "T3B"};
+    const long long n = x.c->bufs.at("T3A").numel;
+    if (8 * n < (long long)kCopyMin) throw Fail("blocks too small");
+    std::vector<double> put[2], back[2];
+    for (int b = 0; b < 2; ++b) {
+        put[b].resize(n);
+        back[b].resize(n);
+        for (long long i = 0; i < n; ++i) put[b][i] = (double)(2 * i + b);
+        if (ccq_b200_block(x.c, name[b], put[b].data(), n, 1)) throw Fail(g_last_error);
+    }
+    slow = true;
+    for (int rep = 0; rep < 20; ++rep) {
+        std::thread th[2];
+        for (int b = 0; b < 2; ++b) {
+            std::fill(back[b].begin(), back[b].end(), -1.0);
+            th[b] = std::thread([&, b] { ccq_b200_block(x.c, name[b], back[b].data(), n, 0); });
+        }
+        for (auto &t : th) t.join();
+        for (int b = 0; b < 2; ++b)
+            if (back[b] != put[b]) throw Fail("a thread read the other's data");
+    }
+    slow = false;
+    return "";
+}
+
 }  // namespace
 
 int main() {
@@ -331,10 +365,15 @@ int main() {
             std::stringstream ss(line);
             std::string cmd, method, out;
             long long froz, oa, ob, orbs, rhf, ao, av, deep;
-            ss >> cmd >> method >> froz >> oa >> ob >> orbs >> rhf >> ao >> av >> deep;
-            Context x(method, froz, oa, ob, orbs, rhf != 0, ao, av);
-            const auto r = run_ranges(x.c);
-            for (size_t k = 0; k + 1 < r.size(); ++k) out += check(x.c, r[k], r[k + 1], deep != 0);
+            ss >> cmd;
+            if (cmd == "copies") {
+                out = copies();
+            } else {
+                ss >> method >> froz >> oa >> ob >> orbs >> rhf >> ao >> av >> deep;
+                Context x(method, froz, oa, ob, orbs, rhf != 0, ao, av);
+                const auto r = run_ranges(x.c);
+                for (size_t k = 0; k + 1 < r.size(); ++k) out += check(x.c, r[k], r[k + 1], deep != 0);
+            }
             std::cout << "ok" << out << std::endl;
         } catch (const std::exception &e) {
             std::cout << "bad " << e.what() << std::endl;

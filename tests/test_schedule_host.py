@@ -68,3 +68,8 @@ def test_items_of_shared_launches(ask, method, froz, occ_a, occ_b, orbs, rhf, ac
 ])
 def test_every_element_is_ordered(ask, method, froz, occ_a, occ_b, orbs, rhf, active):
     assert ask(_sched(method, froz, occ_a, occ_b, orbs, rhf, active, True)).startswith('ok')
+
+
+def test_two_threads_read_one_context(ask):
+    """Large pageable blocks go through pinned slots of the context: one copy at a time."""
+    assert ask('copies') == 'ok'
