@@ -177,7 +177,8 @@ def test_left_ranges(norb, occ_a, occ_b, rhf):
         t0 = {b: ctx.get_block(b, shapes[b]) for b in T12}
         ctx.lambda_init(res[0][0][1] if mode else e[1])
         hist = e + [ctx.lambda_iterate(it)[0] for it in (1, 2)]
-        lam = {b.replace('T', 'L'): ctx.get_block(b.replace('T', 'L'), shapes[b]) for b in T12}
+        parts = np.split(ctx.get_l(), np.cumsum([np.prod(shapes[b]) for b in T12])[:-1])
+        lam = {b.replace('T', 'L'): x for b, x in zip(T12, parts)}
         res.append((np.array(hist), lam, ctx.crcc23()))
     _assert_same(res[0][:2], [r[:2] for r in res[1:]])
     assert np.all(np.abs(res[0][2]) > 0)
