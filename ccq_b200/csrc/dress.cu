@@ -4,7 +4,8 @@
 //   ket:  M[r.] += sum_e t1[r,e] M[e.] for occupied r;   M[.s] += sum_f t2[s,f] M[.f] for occupied s
 // As a copy and four contractions in place, each of the five launches reads and writes the whole n^4 block (or the
 // slice it changes) and waits for the one before: at n = 48, 9 occupied, 17 us for the copy and 21-29 us for each
-// transform, 117 us in all, three times per sweep and at its head.  Two passes read and write the block once each: 65 us.
+// transform, 117 us in all, for three blocks at the head of a sweep (and again before T1B of an open shell, and before T3
+// of CCSDT).  Two passes read and write the block once each: 65 us.
 // One B200, six CCSD iterations: 48 orbitals 4.43 -> 3.62 ms, 32 active orbitals (open shell) 2.00 -> 1.63 ms.  Blocks
 // below 8 MiB (n < 32) keep the separate transforms: there these share launches with the other small contractions,
 // and the three launches per block cost what they save or more (24 orbitals 6.89 against 6.90 ms, 13 orbitals 1.88

@@ -170,7 +170,6 @@ struct __align__(16) MultiItem {
     double alpha;
     int m, n, k, flags;
 };
-inline bool multi_is64(const MultiItem &it) { return it.flags >> MI_SHAPE >= MS_64 && it.flags >> MI_SHAPE < MS_VEC; }
 void launch_gett_multi(const MultiItem *items, int n, bool tiles64, cudaStream_t s);   // items of one kind
 cudaError_t preload_multi();
 

@@ -350,8 +350,8 @@ struct ccq_b200_ctx {
     T3ActGeom geom{};
     double *cvec = nullptr;
     SplitWorkspace split{};
-    // further slicing workspaces: split GETTs take them in turn, so that a split GETT is a node of the sweep's
-    // dependency graph (waiting only for the previous user of its workspace) instead of a barrier
+    // further slicing workspaces: split GETTs take them in turn, so that a split GETT waits only for the previous user
+    // of its own (with one workspace, for the last split GETT)
     std::vector<SplitWorkspace> split_pool;
     // host round trip of ccq_b200_iterate_host: each t_vec block is copied to host_out as soon as its
     // last write of the sweep is done (copy stream cstream, joined into the sweep's stream at its end)
@@ -3627,7 +3627,7 @@ int ccq_b200_set_precision(ccq_b200_ctx *c, int64_t mode, int64_t nslices) {
                 }
             const SplitSizes sz{ma, mb, mc};
             split_reserve(c->split, sz, (int)nslices);
-            // kSplitPool workspaces in turn when they are small (else one, and split GETTs stay barriers)
+            // kSplitPool workspaces in turn when they are small (else one, and each split GETT waits for the last)
             const long long bytes = (ma + mb) * nslices + 8 * mc;
             const int pool = bytes <= kSplitPoolBytes ? kSplitPool : 1;
             for (auto &w : c->split_pool) split_free(w);
