@@ -158,7 +158,7 @@ constexpr int MI_SHAPE = 8;    // flags >> MI_SHAPE: tile shape, below
 // 0..3: one warp's tile is 16 x 16, 32 x 8, 32 x 16, 16 x 32; 4..7: 64 x 64 of a block (+2: A k-major, +1: B
 // k-major); 8: one column (n = 1) and a few k; 9: copy or zero
 constexpr int MS_64 = 4, MS_VEC = 8, MS_COPY = 9;
-constexpr int MULTI_VEC_ROWS = 512, MULTI_VEC_K = 16;
+constexpr int MULTI_VEC_ROWS = 512, MULTI_VEC_K = 16, MULTI_COPY = 1024;   // rows and k of 8; values of 9
 inline void multi_shape(int shape, int &rows, int &cols) {
     rows = shape == MS_VEC ? MULTI_VEC_ROWS : shape >= MS_64 ? 64 : shape == 0 || shape == 3 ? 16 : 32;
     cols = shape == MS_VEC ? 1 : shape >= MS_64 ? 64 : shape == 1 ? 8 : shape == 3 ? 32 : 16;

@@ -215,20 +215,48 @@ __global__ void __launch_bounds__(MT_THREADS, 7) gett_multi_kernel(const MultiIt
         case 3: multi_tile<1, 4>(it, sm, sa, sb); break;
         case MS_VEC: {
             // one column, a few k: one thread per row, no tile
+            constexpr int R = MULTI_VEC_ROWS / MT_THREADS;
+            int ra[R];
+            double v[R];
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+                const int m = threadIdx.x + u * MT_THREADS;
+                ra[u] = m < it.m ? __ldg(it.am + m) : -1;
+                v[u] = 0.0;
+            }
+            const int rb = __ldg(it.bn);
             gdc_wait();
-            for (int m = threadIdx.x; m < it.m; m += MT_THREADS) {
-                const long long ra = __ldg(it.am + m), rb = __ldg(it.bn);
-                double v = 0.0;
-                for (int k = 0; k < it.k; ++k)
-                    v += it.A[ra + __ldg(it.ak + k)] * it.B[rb + __ldg(it.bk + k)];
-                put(it.C + __ldg(it.cm + m) + __ldg(it.cn), it.alpha * v, it.flags & MI_ADD);
+            // all rows' loads before the first store, which an ordinary load may not pass (row by row, and value by
+            // value in the copies below: CCSD at 33 orbitals 1.52 against 1.46 ms, CCSDT at 24 orbitals 6.02 / 5.87 ms)
+            for (int k = 0; k < it.k; ++k) {
+                const int ka = __ldg(it.ak + k);
+                const double b = it.B[(long long)rb + __ldg(it.bk + k)];
+#pragma unroll
+                for (int u = 0; u < R; ++u)
+                    if (ra[u] >= 0) v[u] += it.A[(long long)ra[u] + ka] * b;
+            }
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+                const int m = threadIdx.x + u * MT_THREADS;
+                if (ra[u] >= 0) put(it.C + __ldg(it.cm + m) + __ldg(it.cn), it.alpha * v[u], it.flags & MI_ADD);
             }
             break;
         }
         default: {
-            // copy (A to C) or zero (A null) of m values
+            // copy (A to C) or zero (A null) of m values; the loads first, as above
+            constexpr int R = MULTI_COPY / MT_THREADS;
+            double v[R];
             gdc_wait();
-            for (int i = threadIdx.x; i < it.m; i += MT_THREADS) it.C[i] = it.A ? it.A[i] : 0.0;
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+                const int i = threadIdx.x + u * MT_THREADS;
+                v[u] = it.A && i < it.m ? it.A[i] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+                const int i = threadIdx.x + u * MT_THREADS;
+                if (i < it.m) it.C[i] = v[u];
+            }
         }
     }
 }

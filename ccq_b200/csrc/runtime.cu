@@ -2270,11 +2270,11 @@ Sched build_sched(ccq_b200_ctx *c, size_t from, size_t to) {
             } else {
                 const DevBuf &d = c->bufs.at(o.arg0);
                 const double *src = o.kind == OP_COPY ? c->bufs.at(o.arg1).ptr : nullptr;
-                for (long long x = 0, ne = std::max(d.numel, 1LL); x < ne; x += 1024) {
+                for (long long x = 0, ne = std::max(d.numel, 1LL); x < ne; x += MULTI_COPY) {
                     MultiItem it{};
                     it.A = src ? src + x : nullptr;
                     it.C = d.ptr + x;
-                    it.m = (int)std::min(1024LL, ne - x);
+                    it.m = (int)std::min<long long>(MULTI_COPY, ne - x);
                     it.flags = MS_COPY << MI_SHAPE;
                     items.push_back(it);
                 }
