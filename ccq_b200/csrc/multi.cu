@@ -12,7 +12,8 @@
 // the four warps take them in turn (a chain of DMMAs on one scheduler takes 64 clocks each) and add up through shared
 // memory; with one or two, each warp has its own rows.  Where a contraction's 64 x 64 tiles fill most of the chip they
 // are used instead (gett_multi64_kernel).  Items of one output add with reductions (the output starts at zero or
-// holds earlier terms), so a contraction's K ranges and the terms of one sum need no order among themselves.
+// holds earlier terms), so a contraction's K ranges and the terms of one sum need no order among themselves; an item that
+// overwrites is the only one of its output tile.
 //
 // One B200, a pass of six iterations, one launch per contraction -> shared launches: CCSD of 8 orbitals 1.98 ->
 // 1.08 ms (138 -> 28 launches per sweep), 20 orbitals 2.33 -> 1.34 ms, eight CCSD systems of 16 to 30 orbitals at
